@@ -197,8 +197,8 @@ PTB_API void PTB_EnginePoolStats(uint64_t* counts, int n);
  * per engine and tuned class. Returns the entries written. */
 PTB_API int PTB_MleMappings(int* entries, int n);
 
-/* Fit arithmetic for the Gaussian least-squares modes 1-4. 0 (default): FP64, one thread per ROI, in the
- * reference's exact order of operations (same iteration path as the reference); 1: FP32 iterations, one warp per
+/* Fit arithmetic for the Gaussian least-squares modes 1-4. 0 (default): FP64 in the reference's exact
+ * order of operations (same iteration path as the reference); 1: FP32 iterations, one warp per
  * ROI, with an FP64 re-fit of every ROI whose FP32 run did not stop cleanly; 2: FP64, one warp per ROI.
  * Returns the previous setting. */
 PTB_API int PTB_SetFitPrecision(int mode);

@@ -546,10 +546,8 @@ bool Engine::EnqueueChunk(int slot, const uint16_t* dImg, int H, int W, int B, d
 	};
 	FitParams fpr = fp;
 	const bool hooked = fitHook_ && fpr.mode >= kMleGauss;  // the fit runs in the hook's stage, outside this chain
-	if (fpr.mode >= kMleGauss && !hooked) {
-		if (fpr.lanes == 0) { TunedMapping(fpr, SizeClass(B, H, W)); }
-		fpr.mle.queue = ws.cnt->queue;  // this slot's work-queue counters
-	}
+	if (fpr.mode >= kMleGauss && !hooked && fpr.lanes == 0) { TunedMapping(fpr, SizeClass(B, H, W)); }
+	if (fpr.mode >= kG2Fixed && !hooked) { fpr.mle.queue = ws.cnt->queue; }  // this slot's work-queue counters
 	const bool tune = !hooked && fpr.mode >= kMleGauss && fpr.lanes == 0;  // first chunk of this class: time the mappings
 	pendMleProf_ = prof && fpr.mode >= kMleGauss && !hooked;
 	bool ok = true;
@@ -1006,7 +1004,7 @@ void Engine::MleEvaluations(uint64_t* out, int n)
 
 bool Engine::UploadSpline(FitParams& fp, const std::vector<double>& spline)
 {
-	if (fp.mode >= kMleGauss) {
+	if (fp.mode >= kG2Fixed) {
 		// [0] FP64 re-factorisation count, [1..2] work-queue counters of the persistent fit kernels
 		if (!fallbacks_ && !PTB_CUDA(cudaMalloc(&fallbacks_, 4 * sizeof(unsigned int)))) { return false; }
 		fp.mle.fallbacks = static_cast<unsigned int*>(fallbacks_);

@@ -558,7 +558,7 @@ bool LaunchExactFit(const uint16_t* img, int H, int W, long long N, const Cand* 
                     uint32_t cap, const FitParams& fp, double* rows, const uint8_t* only, cudaStream_t st);
 
 // Fits `n` candidates (device count *nptr, or nconst when nptr is null; `cap` bounds it) into rows[k * 18].
-// precision 0: FP64 in the reference's order (thread per ROI); 1: FP32 warp-per-ROI first, then the FP64 exact
+// precision 0: FP64 in the reference's order; 1: FP32 warp-per-ROI first, then the FP64 exact
 // kernel for the candidates the FP32 pass flags; 2: FP64 warp-per-ROI.
 bool LaunchFit(const uint16_t* img, int H, int W, long long N, const Cand* cands, const uint32_t* nptr, uint32_t nconst,
                uint32_t cap, const FitParams& fp, double* rows, uint8_t* flags, int precision, cudaStream_t st)

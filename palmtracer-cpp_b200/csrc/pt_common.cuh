@@ -138,7 +138,8 @@ struct MleParams {
 	const float* table;        // mode 8: cell-major [cell][64], FP32 (FP32 phases)
 	const double* table64;     // mode 8: the same in FP64 (FP64 phases)
 	unsigned int* fallbacks;   // FP64 Cholesky re-factorisations (diagnostics)
-	unsigned int* queue;       // 2 work-queue counters of the persistent fit kernels (zeroed by the launch), or null
+	unsigned int* queue;       // 2 work-queue counters of the persistent fit kernels (zeroed by the launch), or null;
+	                           // modes 1-4 use the first
 	unsigned long long* evals; // profiling, or null: model evaluations [FP32 LM, FP32 polish, FP64 pre-scan + final]
 };
 

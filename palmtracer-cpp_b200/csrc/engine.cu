@@ -1050,23 +1050,28 @@ bool Engine::UploadSpline(FitParams& fp, const std::vector<double>& spline)
 		splineCacheMode_ = fp.mode;
 		return true;
 	}
-	// cell-major copy of the reference's [64][cell] table: one pixel's 64 coefficients become contiguous
+	// the reference's [64][z][y][x] table with x and y exchanged: the spline fit's lanes read consecutive y cells
 	const size_t cells = static_cast<size_t>(fp.splineSize);
 	if (same) {
 		fp.coeffs = static_cast<const double*>(spline_);
 		return true;
 	}
-	std::vector<double> aos(cells * 64);
-	for (size_t i = 0; i < 64; ++i) {
-		for (size_t c = 0; c < cells; ++c) { aos[c * 64 + i] = spline[i * cells + c]; }
+	std::vector<double> table(cells * 64);
+	const size_t sx = static_cast<size_t>(fp.sx), sy = static_cast<size_t>(fp.sy), slabs = 64 * static_cast<size_t>(fp.sz);
+	for (size_t k = 0; k < slabs; ++k) {
+		const double* src = spline.data() + k * sx * sy;
+		double* dst = table.data() + k * sx * sy;
+		for (size_t y = 0; y < sy; ++y) {
+			for (size_t x = 0; x < sx; ++x) { dst[x * sy + y] = src[y * sx + x]; }
+		}
 	}
-	const size_t bytes = aos.size() * sizeof(double);
+	const size_t bytes = table.size() * sizeof(double);
 	if (bytes > splineBytes_) {
 		if (spline_) { cudaFree(spline_); spline_ = nullptr; splineBytes_ = 0; }
 		if (!PTB_CUDA(cudaMalloc(&spline_, bytes))) { return false; }
 		splineBytes_ = bytes;
 	}
-	if (!PTB_CUDA(cudaMemcpyAsync(spline_, aos.data(), bytes, cudaMemcpyHostToDevice, stream_))) { return false; }
+	if (!PTB_CUDA(cudaMemcpyAsync(spline_, table.data(), bytes, cudaMemcpyHostToDevice, stream_))) { return false; }
 	if (!PTB_CUDA(cudaStreamSynchronize(stream_))) { return false; }
 	fp.coeffs = static_cast<const double*>(spline_);
 	splineCache_ = spline;

@@ -8,8 +8,14 @@
 // carry CRLB values (Offset = CRLB(bg), Intensity/Amplitude = CRLB(A), QualityXY = mean CRLB(x, y), QualityZ =
 // deltaZ * CRLB(z)).
 //
-// The coefficient table is stored cell-major on the device ([cell][64], transposed from the reference's [64][cell])
-// so that the 64 coefficients one pixel needs are one contiguous 512-byte run.
+// The coefficient table lies on the device as [64][z][x][y] (the reference's [64][z][y][x] with x and y exchanged): all
+// pixels of an evaluation share the 64 weights and differ in their cell only, and the lanes of a warp hold consecutive
+// columns of the ROI, which are consecutive y cells. A load of one coefficient then reads 4-5 cache lines per warp. With
+// the 64 coefficients of a cell in one run every lane read its own line: 32 tag lookups per load, which bound the
+// kernel (2 347 ROIs of 9 x 9, table 17 x 17 x 41: 6.3 ms; with this layout 2.4 ms). What bounds it now is the serial
+// part of an iteration (about 25 dependent divisions of the solve and the steps) beside the 64 x 4 products per pixel;
+// three pixels per lane are evaluated side by side so that a coefficient's weights are read once for all of them, held
+// to 168 registers: 3 140 ROIs 2.24 ms, 31 432 21.0 ms (before 6.35 and 60.2; with 128 registers 2.68 and 20.2).
 #include <algorithm>
 
 #include "pt_common.cuh"
@@ -28,8 +34,9 @@ __device__ __forceinline__ double WarpSumD(double v)
 	return v;
 }
 
-struct Patch {
-	double f[64], dx[64], dy[64], dz[64];
+// Weights of the value and of its derivatives in x, y and z, per coefficient.
+struct __align__(16) Patch {
+	double2 fx[64], yz[64];
 };
 
 // Monomial weights x^k y^j z^i and their derivatives (SplineFit.cpp:296-318), two entries per lane.
@@ -43,14 +50,13 @@ __device__ void PatchWeights(Patch& P, double x, double y, double z)
 		for (int a = 0; a < j; ++a) { cy *= y; }
 		for (int a = 0; a < k; ++a) { cxm = cx; cx *= x; }
 		const double zy = cz * cy;
-		P.f[id] = zy * cx;
-		P.dx[id] = k > 0 ? static_cast<double>(k) * (zy * cxm) : 0.0;
+		P.fx[id] = make_double2(zy * cx, k > 0 ? static_cast<double>(k) * (zy * cxm) : 0.0);
 		// derivative in y: j * x^k y^(j-1) z^i; in z: i * x^k y^j z^(i-1)
 		double cym = 1.0, czm = 1.0;
 		for (int a = 0; a + 1 < j; ++a) { cym *= y; }
 		for (int a = 0; a + 1 < i; ++a) { czm *= z; }
-		P.dy[id] = j > 0 ? static_cast<double>(j) * (cz * cym * cx) : 0.0;
-		P.dz[id] = i > 0 ? static_cast<double>(i) * (czm * cy * cx) : 0.0;
+		P.yz[id] = make_double2(j > 0 ? static_cast<double>(j) * (cz * cym * cx) : 0.0,
+		                        i > 0 ? static_cast<double>(i) * (czm * cy * cx) : 0.0);
 	}
 	__syncwarp();
 }
@@ -58,27 +64,56 @@ __device__ void PatchWeights(Patch& P, double x, double y, double z)
 // size_t semantics of Vec3I::Clamp: a negative index wraps and clamps to the upper bound.
 __device__ __forceinline__ long long ClampCell(long long v, int dim) { return (v < 0 || v > dim - 1) ? dim - 1 : v; }
 
-// Model and derivatives at one ROI pixel (SplineFit.cpp:219-240).
-__device__ __forceinline__ double Eval(const FitParams& fp, const Patch& P, long long cx, long long cy, long long cz,
-                                       const double* p, double dudt[5])
+// Pixels a lane evaluates side by side: each coefficient's weights are read from shared memory once for all of them.
+constexpr int kSide = 3;
+
+// Models and derivatives at the lane's pixels idx0, idx0 + 32, .. (those below npx; the others repeat the last pixel),
+// SplineFit.cpp:219-240.
+__device__ __forceinline__ void Eval(const FitParams& fp, const Patch& P, int idx0, int npx, int roi, long long xi, long long yi,
+                                     long long zi, const double* p, double (&model)[kSide], double (&dudt)[kSide][5])
 {
-	const long long x = ClampCell(cx, fp.sx), y = ClampCell(cy, fp.sy), z = ClampCell(cz, fp.sz);
-	const double* c = fp.coeffs + (((z * fp.sy) + y) * fp.sx + x) * 64;
-	double s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-	#pragma unroll 8
-	for (int i = 0; i < 64; ++i) {
-		const double v = __ldg(c + i);
-		s1 += P.f[i] * v;
-		s2 += P.dx[i] * v;
-		s3 += P.dy[i] * v;
-		s4 += P.dz[i] * v;
+	const double* c[kSide];
+	double s1[kSide], s2[kSide], s3[kSide], s4[kSide];
+	const long long z = ClampCell(zi, fp.sz);
+	#pragma unroll
+	for (int t = 0; t < kSide; ++t) {
+		const int idx = min(idx0 + 32 * t, npx - 1);
+		const int i = idx / roi, j = idx - i * roi;
+		const long long x = ClampCell(xi + i + fp.offsetXY, fp.sx), y = ClampCell(yi + j + fp.offsetXY, fp.sy);
+		c[t] = fp.coeffs + ((z * fp.sx) + x) * fp.sy + y;
+		s1[t] = s2[t] = s3[t] = s4[t] = 0;
 	}
-	dudt[0] = 1;
-	dudt[1] = s1;
-	dudt[2] = s2 * (-1 * p[1]);
-	dudt[3] = s3 * (-1 * p[1]);
-	dudt[4] = s4 * p[1];
-	return p[0] + (p[1] * dudt[1]);
+	constexpr int kBatch = 8;
+	#pragma unroll 1
+	for (int i0 = 0; i0 < 64; i0 += kBatch) {
+		double v[kSide][kBatch];
+		#pragma unroll
+		for (int t = 0; t < kSide; ++t) {
+			#pragma unroll
+			for (int i = 0; i < kBatch; ++i) { v[t][i] = __ldg(c[t] + i * fp.splineSize); }
+			c[t] += kBatch * fp.splineSize;
+		}
+		#pragma unroll
+		for (int i = 0; i < kBatch; ++i) {
+			const double2 fx = P.fx[i0 + i], yz = P.yz[i0 + i];
+			#pragma unroll
+			for (int t = 0; t < kSide; ++t) {
+				s1[t] += fx.x * v[t][i];
+				s2[t] += fx.y * v[t][i];
+				s3[t] += yz.x * v[t][i];
+				s4[t] += yz.y * v[t][i];
+			}
+		}
+	}
+	#pragma unroll
+	for (int t = 0; t < kSide; ++t) {
+		dudt[t][0] = 1;
+		dudt[t][1] = s1[t];
+		dudt[t][2] = s2[t] * (-1 * p[1]);
+		dudt[t][3] = s3[t] * (-1 * p[1]);
+		dudt[t][4] = s4[t] * p[1];
+		model[t] = p[0] + (p[1] * dudt[t][1]);
+	}
 }
 
 __device__ void StoreRow(double* row, double segI, double surf, double x, double y, double z, double off, double amp,
@@ -100,7 +135,7 @@ __device__ void StoreRow(double* row, double segI, double surf, double x, double
 	}
 }
 
-__global__ void __launch_bounds__(32 * kWarps) SplineFitKernel(const uint16_t* __restrict__ img, int H, int W, long long N,
+__global__ void __launch_bounds__(32 * kWarps, 3) SplineFitKernel(const uint16_t* __restrict__ img, int H, int W, long long N,
                                                                 const Cand* __restrict__ cands, const uint32_t* nptr,
                                                                 uint32_t nconst, FitParams fp, double* rows)
 {
@@ -172,19 +207,24 @@ __global__ void __launch_bounds__(32 * kWarps) SplineFitKernel(const uint16_t* _
 			long long xi, yi, zi;
 			cell(p, xi, yi, zi);
 			double dev = 0, jac[5] = {0, 0, 0, 0, 0}, hs[15] = {};
-			for (int idx = lane; idx < npx; idx += 32) {
-				const int i = idx / roi, j = idx - i * roi;
-				const double d = static_cast<double>(__ldg(base + static_cast<long long>(i) * W + j));
-				double dudt[5];
-				const double model = Eval(fp, P, xi + i + fp.offsetXY, yi + j + fp.offsetXY, zi, p, dudt);
-				dev += d > 0 ? 2 * (model - d - (d * log(model / d))) : 2 * model;
-				const double t1 = 1 - (d / model), t2 = d / (model * model);
-				int q = 0;
+			for (int idx0 = lane; idx0 < npx; idx0 += 32 * kSide) {
+				double dudt[kSide][5], model[kSide];
+				Eval(fp, P, idx0, npx, roi, xi, yi, zi, p, model, dudt);
 				#pragma unroll
-				for (int a = 0; a < 5; ++a) {
-					jac[a] += t1 * dudt[a];
+				for (int t = 0; t < kSide; ++t) {
+					const int idx = idx0 + 32 * t;
+					if (idx >= npx) { break; }
+					const int i = idx / roi, j = idx - i * roi;
+					const double d = static_cast<double>(__ldg(base + static_cast<long long>(i) * W + j));
+					dev += d > 0 ? 2 * (model[t] - d - (d * log(model[t] / d))) : 2 * model[t];
+					const double t1 = 1 - (d / model[t]), t2 = d / (model[t] * model[t]);
+					int q = 0;
 					#pragma unroll
-					for (int b = a; b < 5; ++b) { hs[q++] += t2 * dudt[a] * dudt[b]; }
+					for (int a = 0; a < 5; ++a) {
+						jac[a] += t1 * dudt[t][a];
+						#pragma unroll
+						for (int b = a; b < 5; ++b) { hs[q++] += t2 * dudt[t][a] * dudt[t][b]; }
+					}
 				}
 			}
 			err = err + WarpSumD(dev);
@@ -264,15 +304,18 @@ __global__ void __launch_bounds__(32 * kWarps) SplineFitKernel(const uint16_t* _
 		long long xi, yi, zi;
 		cell(p, xi, yi, zi);
 		double fs[15] = {};
-		for (int idx = lane; idx < npx; idx += 32) {
-			const int i = idx / roi, j = idx - i * roi;
-			double dudt[5];
-			const double model = Eval(fp, P, xi + i + fp.offsetXY, yi + j + fp.offsetXY, zi, p, dudt);
-			int q = 0;
+		for (int idx0 = lane; idx0 < npx; idx0 += 32 * kSide) {
+			double dudt[kSide][5], model[kSide];
+			Eval(fp, P, idx0, npx, roi, xi, yi, zi, p, model, dudt);
 			#pragma unroll
-			for (int a = 0; a < 5; ++a) {
+			for (int t = 0; t < kSide; ++t) {
+				if (idx0 + 32 * t >= npx) { break; }
+				int q = 0;
 				#pragma unroll
-				for (int b = a; b < 5; ++b) { fs[q++] += dudt[b] * dudt[a] / model; }
+				for (int a = 0; a < 5; ++a) {
+					#pragma unroll
+					for (int b = a; b < 5; ++b) { fs[q++] += dudt[t][b] * dudt[t][a] / model[t]; }
+				}
 			}
 		}
 		double m[25];

@@ -156,7 +156,7 @@ struct FitParams {
 	long long splineSize;  // sx * sy * sz
 	long long offsetXY;
 	double roiParam, initZ, deltaZ, intensityRatio;
-	const double* coeffs;  // device, cell-major [cell][64]
+	const double* coeffs;  // device, [64][sz][sx][sy]
 	MleParams mle;         // modes 6-8
 	int lanes;             // ROI mapping for modes 6-8: 1 thread per ROI, else warp per ROI (autotuned)
 	cudaEvent_t* marks;    // profiling, or null: 5 events recorded around the phases of the modes 6-8 fit

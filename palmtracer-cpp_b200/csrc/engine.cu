@@ -167,6 +167,32 @@ uint32_t IndepBound(int H, int W) { return static_cast<uint32_t>(((H + 1) / 2)) 
 
 }  // namespace
 
+cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
+{
+	constexpr int kDevices = 64;
+	static std::mutex mu;
+	static cudaMemPool_t pools[kDevices] = {};
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess || dev < 0 || dev >= kDevices) { return e != cudaSuccess ? e : cudaErrorInvalidDevice; }
+	cudaMemPool_t pool = nullptr;
+	{
+		std::lock_guard<std::mutex> lock(mu);
+		if (pools[dev] == nullptr) {
+			cudaMemPoolProps props{};
+			props.allocType = cudaMemAllocationTypePinned;
+			props.location.type = cudaMemLocationTypeDevice;
+			props.location.id = dev;
+			e = cudaMemPoolCreate(&pools[dev], &props);
+			uint64_t keep = kScratchKeep;
+			if (e == cudaSuccess) { e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep); }
+			if (e != cudaSuccess) { return e; }
+		}
+		pool = pools[dev];
+	}
+	return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
 // Host memcpy over several threads (pageable buffers go through pinned staging; one thread copies about 10 GB/s).
 void ParallelCopy(void* dst, const void* src, size_t bytes)
 {
@@ -1121,9 +1147,9 @@ long long Engine::FitPositions(const uint16_t* input, const double* positions, u
 	Cand* dCand = nullptr;
 	double* dRows = nullptr;
 	uint8_t* dFlag = nullptr;
-	bool ok = PTB_CUDA(cudaMallocAsync(&dCand, sizeof(Cand) * nPoints, stream_));
-	ok = ok && PTB_CUDA(cudaMallocAsync(&dRows, sizeof(double) * kCols * nPoints, stream_));
-	ok = ok && PTB_CUDA(cudaMallocAsync(&dFlag, nPoints, stream_));
+	bool ok = PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dCand), sizeof(Cand) * nPoints, stream_));
+	ok = ok && PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dRows), sizeof(double) * kCols * nPoints, stream_));
+	ok = ok && PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dFlag), nPoints, stream_));
 	ok = ok && PTB_CUDA(cudaMemcpyAsync(dCand, cands.data(), sizeof(Cand) * nPoints, cudaMemcpyHostToDevice, stream_));
 	// modes 6-8: a warp per ROI while the points fill the GPU a few times at most (shortest call), else a thread per ROI
 	if (fp.mode >= kMleGauss && fp.lanes == 0) { fp.lanes = nPoints <= 148ull * 64 ? 32 : 1; }
@@ -1159,7 +1185,7 @@ bool Engine::Planes(const uint16_t* input, double* output, uint64_t height, uint
 	const uint64_t B = std::max<uint64_t>(1, std::min<uint64_t>(planes, budget_ / perFrame));
 	if (!ReserveImage(N * B * sizeof(uint16_t))) { return false; }
 	double* dOut = nullptr;
-	if (!PTB_CUDA(cudaMallocAsync(&dOut, N * B * sizeof(double), stream_))) { return false; }
+	if (!PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dOut), N * B * sizeof(double), stream_))) { return false; }
 	bool ok = true;
 	for (uint64_t z0 = 0; z0 < planes && ok; z0 += B) {
 		const uint64_t b = std::min<uint64_t>(B, planes - z0);
@@ -1233,8 +1259,8 @@ bool Engine::Track(const double* input, uint64_t* output, uint64_t n, double max
 	if (!Init()) { return false; }
 	double* dIn = nullptr;
 	uint64_t* dOut = nullptr;
-	bool ok = PTB_CUDA(cudaMallocAsync(&dIn, n * 4 * sizeof(double), stream_));
-	ok = ok && PTB_CUDA(cudaMallocAsync(&dOut, n * 2 * sizeof(uint64_t), stream_));
+	bool ok = PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dIn), n * 4 * sizeof(double), stream_));
+	ok = ok && PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dOut), n * 2 * sizeof(uint64_t), stream_));
 	ok = ok && PTB_CUDA(cudaMemcpyAsync(dIn, input, n * 4 * sizeof(double), cudaMemcpyHostToDevice, stream_));
 	ok = ok && TrackDevice(dIn, dOut, n, maxDistance, stream_);
 	ok = ok && PTB_CUDA(cudaMemcpyAsync(output, dOut, n * 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream_));
@@ -1250,8 +1276,8 @@ bool Engine::AstigEstimate(const double* input, double* output, uint64_t n, doub
 	const size_t bytes = static_cast<size_t>(n) * 2 * sizeof(double);
 	double* dIn = nullptr;
 	double* dOut = nullptr;
-	bool ok = PTB_CUDA(cudaMallocAsync(&dIn, bytes, stream_));
-	ok = ok && PTB_CUDA(cudaMallocAsync(&dOut, bytes, stream_));
+	bool ok = PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dIn), bytes, stream_));
+	ok = ok && PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dOut), bytes, stream_));
 	ok = ok && PTB_CUDA(cudaMemcpyAsync(dIn, input, bytes, cudaMemcpyHostToDevice, stream_));
 	ok = ok && LaunchAstigEstimate(dIn, dOut, n, pixelSize, model, zMax, stream_);
 	ok = ok && PTB_CUDA(cudaMemcpyAsync(output, dOut, bytes, cudaMemcpyDeviceToHost, stream_));

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -61,6 +62,13 @@ const std::string& LastError();
 void ClearError();
 bool CheckCuda(cudaError_t e, const char* what, const char* file, int line);
 void CountLaunch(uint64_t n = 1);
+
+// Device scratch of one call, ordered on `st` (freed with cudaFreeAsync on a stream that follows its last use). It comes
+// from a pool of its own per device that keeps up to kScratchKeep bytes between calls; the default pool returns its
+// memory at every synchronisation, and mapping it again for each call took longer than the calls' kernels (tracking of
+// 396 000 points on the device: 1.53 ms, with this pool 0.46 ms).
+constexpr size_t kScratchKeep = 1ull << 30;
+cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st);
 
 #define PTB_CUDA(call) ::ptb::CheckCuda((call), #call, __FILE__, __LINE__)
 #define PTB_LAUNCHED() ::ptb::CheckCuda(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)

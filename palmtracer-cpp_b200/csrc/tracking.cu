@@ -13,9 +13,12 @@
 // plane whose X lies within w of its own (binary search, then a forward scan), w slightly above maxDistance. A pair
 // outside the window has fl(dx * dx) > maxDistance^2, so fl(fl(dx^2) + fl(dy^2)) > maxDistance^2 too (rounding is
 // monotone) and the reference rejects it; inside, the reference's own test decides. Two passes, count then emit.
-// Step 3 sorts each transition's pairs in one CTA and links them in order with one thread per transition
-// (transitions touch disjoint successor and predecessor entries); step 4 is a scan over chain heads and pointer
-// jumping along predecessor links. d2 is formed with explicitly rounded FP64 operations (no contraction), so the
+// Step 3 links, round by round, every pair that comes first in the order both among the pairs its source could still
+// take and among those its target could: no earlier pair can claim either end any more, so the sequential pass links it
+// too, and what it leaves is the same problem on fewer points (TrackMatch, one CTA per transition, no sorting). A
+// transition that is not done after kMatchRounds rounds (rows of equal distances link one pair a round) is finished by
+// the sequential pass: its pairs sorted in one CTA and linked in order by one thread. Step 4 is a scan over chain heads
+// and pointer jumping along predecessor links. d2 is formed with explicitly rounded FP64 operations (no contraction), so the
 // admitted pairs and their order are the reference's; ties in (Plane, Id), which the reference's unstable sort
 // leaves unspecified, are ordered by input index.
 #include <algorithm>
@@ -59,10 +62,24 @@ __global__ void TrackKeys(const double* __restrict__ in, uint32_t n, uint64_t* p
 	}
 }
 
+// The lanes of the calling warp that hold the same plane: their number and this lane's rank among them; true in the
+// first of them. Tables mostly list a plane's points together, so one atomic per warp replaces 32 on one counter
+// (396 000 points on 400 planes: count and scatter 93 and 106 us, now 7 and 7).
+__device__ __forceinline__ bool SamePlane(uint32_t p, uint32_t& rank, uint32_t& peers)
+{
+	const unsigned mask = __match_any_sync(0xffffffffu, p);
+	rank = static_cast<uint32_t>(__popc(mask & ((1u << (threadIdx.x & 31)) - 1u)));
+	peers = static_cast<uint32_t>(__popc(mask));
+	return rank == 0;
+}
+
 __global__ void PlaneCount(const uint64_t* __restrict__ plane, uint32_t n, uint64_t minPlane, uint32_t* count)
 {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		atomicAdd(&count[plane[i] - minPlane], 1u);
+	const uint32_t whole = (n + 31u) & ~31u;  // whole warps
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < whole; i += gridDim.x * blockDim.x) {
+		uint32_t rank, peers;
+		const uint32_t p = i < n ? static_cast<uint32_t>(plane[i] - minPlane) : 0xffffffffu;
+		if (SamePlane(p, rank, peers) && i < n) { atomicAdd(&count[p], peers); }
 	}
 }
 
@@ -70,11 +87,17 @@ __global__ void PlaneCount(const uint64_t* __restrict__ plane, uint32_t n, uint6
 __global__ void PlaneScatter(const uint64_t* __restrict__ plane, const uint64_t* __restrict__ id, uint32_t n, uint64_t minPlane,
                              const uint32_t* __restrict__ begin, uint32_t* cursor, unsigned long long* k1, unsigned long long* k2)
 {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		const uint64_t p = plane[i] - minPlane;
-		const uint32_t pos = begin[p] + atomicAdd(&cursor[p], 1u);
-		k1[pos] = id[i];
-		k2[pos] = i;
+	const uint32_t whole = (n + 31u) & ~31u;  // whole warps
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < whole; i += gridDim.x * blockDim.x) {
+		uint32_t rank, peers, at = 0;
+		const uint32_t p = i < n ? static_cast<uint32_t>(plane[i] - minPlane) : 0xffffffffu;
+		const bool first = SamePlane(p, rank, peers);
+		if (first && i < n) { at = begin[p] + atomicAdd(&cursor[p], peers); }
+		at = __shfl_sync(0xffffffffu, at, __ffs(__match_any_sync(0xffffffffu, p)) - 1);
+		if (i < n) {
+			k1[at + rank] = id[i];
+			k2[at + rank] = i;
+		}
 	}
 }
 
@@ -108,13 +131,16 @@ __device__ void BitonicPairs(unsigned long long* k1, unsigned long long* k2, uin
 
 // One CTA per segment [off[s], off[s + 1]): sorts its (k1, k2) pairs ascending. Segments longer than kSegSmem sort
 // in global scratch at [2 off[s], 2 off[s] + 2 len) (a power of two below 2 len, so segments never overlap).
+// pending (null: every segment): the segments to sort.
 __global__ void __launch_bounds__(kSortThreads) SegmentSort(unsigned long long* k1, unsigned long long* k2, const uint32_t* __restrict__ off,
-                                                            uint32_t nseg, unsigned long long* s1, unsigned long long* s2)
+                                                            uint32_t nseg, unsigned long long* s1, unsigned long long* s2,
+                                                            const uint32_t* __restrict__ pending)
 {
 	extern __shared__ unsigned long long segSmem[];
 	unsigned long long* a1 = segSmem;
 	unsigned long long* a2 = segSmem + kSegSmem;
 	for (uint32_t s = blockIdx.x; s < nseg; s += gridDim.x) {
+		if (pending && !pending[s]) { continue; }
 		const uint32_t b = off[s], len = off[s + 1] - b;
 		if (len <= 1) { continue; }
 		uint32_t p2 = 1;
@@ -228,11 +254,79 @@ __global__ void TransitionOffsets(const uint32_t* __restrict__ begin, const uint
 	for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p <= P; p += gridDim.x * blockDim.x) { off[p] = pairBegin[begin[p]]; }
 }
 
-// One thread per transition: links its ordered pairs greedily (source without successor, target without
-// predecessor). Transitions touch disjoint entries: successors of plane p, predecessors of plane p + 1.
-__global__ void TrackLink(const unsigned long long* __restrict__ k2, const uint32_t* __restrict__ off, uint32_t P, uint32_t* next, uint32_t* prev)
+constexpr int kMatchThreads = 512;
+constexpr int kMatchRounds = 24;
+
+// One CTA per transition p (plane p's points are the sources, plane p + 1's the targets; transitions touch disjoint
+// entries). Each round: every open source offers its distance to every open target in reach, equal distances are
+// settled for the lower source, and a source whose best open target (nearest, then lowest) took its offer links to it.
+// tgtD2 / tgtSrc [n]: a target's best offer, all ones when it has none. pending[p]: 1 when rounds ran out.
+// Bound: L2 latency of a round's three passes over the pairs (a table needs 5-10 rounds). 396 000 points on 400 planes:
+// 32 us, where sorting each transition's pairs and linking them with one thread took 70 + 1562 us.
+__global__ void __launch_bounds__(kMatchThreads) TrackMatch(const unsigned long long* __restrict__ k1, const unsigned long long* __restrict__ k2,
+                                                            const uint32_t* __restrict__ begin, const uint32_t* __restrict__ pairBegin, uint32_t P,
+                                                            unsigned long long* tgtD2, uint32_t* tgtSrc, uint32_t* next, uint32_t* prev,
+                                                            uint32_t* pending)
+{
+	for (uint32_t p = blockIdx.x; p < P; p += gridDim.x) {
+		const uint32_t a = begin[p], b = begin[p + 1];
+		bool again = true;
+		for (int round = 0; round < kMatchRounds && again; ++round) {
+			bool any = false;
+			for (uint32_t k = a + threadIdx.x; k < b; k += kMatchThreads) {
+				if (next[k] != kNoLink) { continue; }
+				for (uint32_t c = pairBegin[k]; c < pairBegin[k + 1]; ++c) {
+					const uint32_t j = static_cast<uint32_t>(k2[c]);
+					if (prev[j] != kNoLink) { continue; }
+					atomicMin(tgtD2 + j, k1[c]);
+					any = true;
+				}
+			}
+			again = __syncthreads_or(any);
+			if (!again) { break; }
+			for (uint32_t k = a + threadIdx.x; k < b; k += kMatchThreads) {
+				if (next[k] != kNoLink) { continue; }
+				for (uint32_t c = pairBegin[k]; c < pairBegin[k + 1]; ++c) {
+					const uint32_t j = static_cast<uint32_t>(k2[c]);
+					if (prev[j] == kNoLink && __ldcg(tgtD2 + j) == k1[c]) { atomicMin(tgtSrc + j, k); }
+				}
+			}
+			__syncthreads();
+			for (uint32_t k = a + threadIdx.x; k < b; k += kMatchThreads) {
+				if (next[k] != kNoLink) { continue; }
+				unsigned long long d2 = ~0ull;
+				uint32_t to = kNoLink;
+				for (uint32_t c = pairBegin[k]; c < pairBegin[k + 1]; ++c) {
+					const uint32_t j = static_cast<uint32_t>(k2[c]);
+					// a target taken in this round has its best offer settled: only its own source links to it, so an
+					// entry of prev that changes meanwhile belongs to a target whose offer this source did not win
+					if (__ldcg(tgtD2 + j) == ~0ull) { continue; }
+					if (k1[c] < d2 || (k1[c] == d2 && j < to)) { d2 = k1[c]; to = j; }
+				}
+				if (to != kNoLink && __ldcg(tgtD2 + to) == d2 && __ldcg(tgtSrc + to) == k) {
+					next[k] = to;
+					prev[to] = k;
+				}
+			}
+			__syncthreads();
+			// the next round's offers start afresh: targets taken keep none
+			for (uint32_t j = begin[p + 1] + threadIdx.x; j < begin[p + 2]; j += kMatchThreads) {
+				tgtD2[j] = ~0ull;
+				tgtSrc[j] = kNoLink;
+			}
+			__syncthreads();
+		}
+		if (threadIdx.x == 0) { pending[p] = again ? 1u : 0u; }
+	}
+}
+
+// One thread per transition left unfinished: links its ordered pairs greedily (source without successor, target
+// without predecessor).
+__global__ void TrackLink(const unsigned long long* __restrict__ k2, const uint32_t* __restrict__ off, const uint32_t* __restrict__ pending,
+                          uint32_t P, uint32_t* next, uint32_t* prev)
 {
 	for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
+		if (!pending[p]) { continue; }
 		for (uint32_t c = off[p]; c < off[p + 1]; ++c) {
 			const uint32_t from = static_cast<uint32_t>(k2[c] >> 32), to = static_cast<uint32_t>(k2[c] & 0xffffffffu);
 			if (next[from] == kNoLink && prev[to] == kNoLink) {
@@ -251,11 +345,21 @@ __global__ void HeadFlags(const uint32_t* __restrict__ prev, uint32_t n, uint32_
 	}
 }
 
-// One pointer-jumping round: root[k] <- root[root[k]] (in place: a thread that reads an already advanced entry only
-// moves further toward the chain head, so the rounds needed are at most those of the synchronous scheme).
+// Pointer jumping, kJumpHops hops per launch: root[k] moves up by at least that many entries or to the chain head (in
+// place: an entry that another thread has already advanced only leads further up). Every launch multiplies the
+// distance covered by at least kJumpHops.
+constexpr int kJumpHops = 32;
 __global__ void Jump(uint32_t* root, uint32_t n)
 {
-	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) { root[k] = root[root[k]]; }
+	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+		uint32_t r = root[k];
+		for (int h = 0; h < kJumpHops; ++h) {
+			const uint32_t up = __ldcg(root + r);
+			if (up == r) { break; }
+			r = up;
+		}
+		root[k] = r;
+	}
 }
 
 __global__ void TrackOutput(const unsigned long long* __restrict__ id, const uint32_t* __restrict__ root, const uint32_t* __restrict__ headRank,
@@ -270,12 +374,12 @@ __global__ void TrackOutput(const unsigned long long* __restrict__ id, const uin
 constexpr size_t kSegSmemBytes = 2 * kSegSmem * sizeof(unsigned long long);
 
 bool LaunchSegmentSort(unsigned long long* k1, unsigned long long* k2, const uint32_t* off, uint32_t nseg, unsigned long long* s1,
-                       unsigned long long* s2, cudaStream_t st)
+                       unsigned long long* s2, cudaStream_t st, const uint32_t* pending = nullptr)
 {
 	static const bool configured = PTB_CUDA(cudaFuncSetAttribute(SegmentSort, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                                             static_cast<int>(kSegSmemBytes)));
 	if (!configured) { return false; }
-	SegmentSort<<<std::max<uint32_t>(1, std::min<uint32_t>(nseg, 148u * 32)), kSortThreads, kSegSmemBytes, st>>>(k1, k2, off, nseg, s1, s2);
+	SegmentSort<<<std::max<uint32_t>(1, std::min<uint32_t>(nseg, 148u * 32)), kSortThreads, kSegSmemBytes, st>>>(k1, k2, off, nseg, s1, s2, pending);
 	CountLaunch();
 	return PTB_LAUNCHED();
 }
@@ -298,7 +402,7 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 	auto alloc = [&](auto*& p, size_t count) {
 		using T = std::remove_pointer_t<std::remove_reference_t<decltype(p)>>;
 		void* v = nullptr;
-		const bool ok = PTB_CUDA(cudaMallocAsync(&v, std::max<size_t>(count, 1) * sizeof(T), st));
+		const bool ok = PTB_CUDA(ScratchAlloc(&v, std::max<size_t>(count, 1) * sizeof(T), st));
 		p = static_cast<T*>(v);
 		if (ok) { bufs.push_back(v); }
 		return ok;
@@ -377,10 +481,11 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 		ok = false;
 	}
 	uint32_t *off = nullptr, *next = nullptr, *prev = nullptr, *head = nullptr, *root = nullptr;
-	unsigned long long *ck1 = nullptr, *ck2 = nullptr, *c1 = nullptr, *c2 = nullptr;
+	unsigned long long *ck1 = nullptr, *ck2 = nullptr, *c1 = nullptr, *c2 = nullptr, *tgtD2 = nullptr;
+	uint32_t *tgtSrc = nullptr, *pending = nullptr;
 	ok = ok && ExclusiveScan(pairBegin, nullptr, n, n + 1, scanScratch, nullptr, st);
 	ok = ok && alloc(ck1, pairs) && alloc(ck2, pairs) && alloc(c1, 2 * pairs) && alloc(c2, 2 * pairs) && alloc(off, P + 1) &&
-	     alloc(next, n) && alloc(prev, n) && alloc(head, n + 2) && alloc(root, n);
+	     alloc(next, n) && alloc(prev, n) && alloc(head, n + 2) && alloc(root, n) && alloc(tgtD2, n) && alloc(tgtSrc, n) && alloc(pending, P);
 	if (ok && pairs > 0) {
 		TrackPairs<true><<<G, kTrackThreads, 0, st>>>(xy, rel, begin, xk1, xk2, n, P, r2, w, pairBegin, nullptr, ck1, ck2);
 		CountLaunch();
@@ -388,12 +493,15 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 	}
 	ok = ok && PTB_CUDA(cudaMemsetAsync(next, 0xff, sizeof(uint32_t) * n, st)) && PTB_CUDA(cudaMemsetAsync(prev, 0xff, sizeof(uint32_t) * n, st));
 	if (ok && pairs > 0) {
+		ok = PTB_CUDA(cudaMemsetAsync(tgtD2, 0xff, sizeof(unsigned long long) * n, st)) &&
+		     PTB_CUDA(cudaMemsetAsync(tgtSrc, 0xff, sizeof(uint32_t) * n, st));
+		TrackMatch<<<std::min<uint32_t>(P, 148u * 32), kMatchThreads, 0, st>>>(ck1, ck2, begin, pairBegin, P, tgtD2, tgtSrc, next, prev, pending);
 		TransitionOffsets<<<Grid(P + 1, kTrackThreads), kTrackThreads, 0, st>>>(begin, pairBegin, P, off);
-		CountLaunch();
-		ok = PTB_LAUNCHED() && LaunchSegmentSort(ck1, ck2, off, P, c1, c2, st);
+		CountLaunch(2);
+		ok = ok && PTB_LAUNCHED() && LaunchSegmentSort(ck1, ck2, off, P, c1, c2, st, pending);
 	}
 	if (ok && pairs > 0) {
-		TrackLink<<<Grid(P, 128), 128, 0, st>>>(ck2, off, P, next, prev);
+		TrackLink<<<Grid(P, 128), 128, 0, st>>>(ck2, off, pending, P, next, prev);
 		CountLaunch();
 		ok = PTB_LAUNCHED();
 	}
@@ -402,9 +510,9 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 		CountLaunch();
 		ok = PTB_LAUNCHED() && ExclusiveScan(head, nullptr, n, n + 1, scanScratch, nullptr, st);
 	}
-	// a chain has at most one point per plane: ceil(log2(P)) + 1 rounds reach every head
+	// a chain has at most one point per plane
 	int rounds = 1;
-	while ((1ull << (rounds - 1)) < P) { ++rounds; }
+	for (unsigned long long reach = kJumpHops; reach < P; reach *= kJumpHops) { ++rounds; }
 	for (int r = 0; ok && r < rounds; ++r) {
 		Jump<<<G, kTrackThreads, 0, st>>>(root, n);
 		CountLaunch();

@@ -160,7 +160,7 @@ namespace {
 
 size_t Align(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
-// Words of the per-chunk frame arrays zeroed before each chunk: five [B + 1] arrays.
+// Words of the per-chunk frame arrays: frameDom, frameSeeds, frameRoute, frameSuspect and frameReflood [B + 1].
 size_t FrameWords(int B) { return 5 * (static_cast<size_t>(B) + 1); }
 
 uint32_t IndepBound(int H, int W) { return static_cast<uint32_t>(((H + 1) / 2)) * static_cast<uint32_t>(((W + 1) / 2)); }
@@ -255,7 +255,6 @@ static size_t PlanWorkspace(Workspace& ws, int H, int W, int B, uint32_t rowsCap
 	take(ws.w1, P);
 	take(ws.par, P);
 	take(ws.lab, P);
-	take(ws.rootmask, rows * g.words);
 	take(ws.rowcnt, rows + 1);
 	take(ws.dom, P);
 	take(ws.seeds, P);
@@ -290,14 +289,6 @@ static size_t PlanWorkspace(Workspace& ws, int H, int W, int B, uint32_t rowsCap
 	take(ws.fuNeighbour, capComp);
 	take(ws.fuBecome, capComp);
 	take(ws.fuLocked, capComp);
-	// frameDom, frameSeeds, frameRoute, frameSuspect and frameReflood (zeroed together for each chunk)
-	take(ws.frameDom, FrameWords(B));
-	if (base) {
-		ws.frameSeeds = ws.frameDom + B + 1;
-		ws.frameRoute = ws.frameSeeds + B + 1;
-		ws.frameSuspect = ws.frameRoute + B + 1;
-		ws.frameReflood = ws.frameSuspect + B + 1;
-	}
 	take(ws.rfVals, static_cast<size_t>(kRefloodSlots) * 2 * kRefloodCap);
 	take(ws.rfGrp, static_cast<size_t>(kRefloodSlots) * 2 * kRefloodCap);
 	take(ws.rfOff, static_cast<size_t>(kRefloodSlots) * 2 * (kRefloodBuckets + 1));
@@ -321,8 +312,17 @@ static size_t PlanWorkspace(Workspace& ws, int H, int W, int B, uint32_t rowsCap
 	take(ws.sortIdx, static_cast<size_t>(ws.capRows) * 2);
 	take(ws.sortKey, static_cast<size_t>(ws.capRows) * 4);
 	take(ws.fitFlag, ws.capRows);
-	take(ws.scanBlock, P / 4096 + 64);
 	take(ws.cnt, 1);
+	take(ws.scanState, ScanStateWords(static_cast<uint32_t>(rows)) + 3 * ScanStateWords(capComp) + ScanStateWords(capComp));
+	take(ws.frameDom, FrameWords(B));
+	if (base) {
+		ws.frameSeeds = ws.frameDom + B + 1;
+		ws.frameRoute = ws.frameSeeds + B + 1;
+		ws.frameSuspect = ws.frameRoute + B + 1;
+		ws.frameReflood = ws.frameSuspect + B + 1;
+	}
+	take(ws.rootmask, rows * g.words);
+	if (base) { ws.zeroBytes = base + off - reinterpret_cast<char*>(ws.cnt); }
 	return off;
 }
 
@@ -585,9 +585,7 @@ bool Engine::EnqueueChunk(int slot, const uint16_t* dImg, int H, int W, int B, d
 	}
 	const uint32_t rowsCap = ws.capRows;
 	auto segmentAndDetect = [&]() {
-		bool k = PTB_CUDA(cudaMemsetAsync(ws.cnt, 0, sizeof(Counters), st));
-		k = k && PTB_CUDA(cudaMemsetAsync(ws.rootmask, 0, sizeof(uint32_t) * static_cast<size_t>(B) * H * ws.g.words, st));
-		k = k && PTB_CUDA(cudaMemsetAsync(ws.frameDom, 0, sizeof(uint32_t) * FrameWords(B), st));
+		bool k = PTB_CUDA(cudaMemsetAsync(ws.cnt, 0, ws.zeroBytes, st));
 		mark(0);
 		k = k && LaunchDetect(ws, thr, st);
 		mark(1);
@@ -674,7 +672,7 @@ long long Engine::CompleteChunk(int slot, uint32_t* truncatedFrames)
 		return -1;
 	}
 	if (c.fault) {
-		SetError("the detection kernel's wait for its staged input tile ran out");
+		SetError("a bounded wait ran out (the detection kernel's for its staged input tile or a prefix sum's for a predecessor)");
 		return -1;
 	}
 	segCounts_[1] += c.nroute;

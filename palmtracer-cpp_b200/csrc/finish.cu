@@ -2,6 +2,8 @@
 //
 // Reference: SegmentationInfo fields from ComputeStatistics (Segmentation2D.cpp:144-175); per-frame sort with
 // std::weak_order on Y then X (FrameProcessor.cpp:35-39); Id / Plane / Index assignment (lib/Palm.cpp:24-43).
+#include <algorithm>
+
 #include "pt_common.cuh"
 
 namespace ptb {
@@ -11,6 +13,7 @@ namespace {
 // Region sums are exact integers in 2^-16 units, so x = sum(v j) / sum(v) is the reference's FP64 quotient exactly.
 __global__ void BuildCandidates(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->nfit, ws.capRows);
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		const uint32_t r = ws.candRegion[k];
@@ -69,8 +72,9 @@ __device__ void Bitonic(unsigned long long* ky, unsigned long long* kx, uint32_t
 }
 
 // One CTA per frame: sort that frame's rows by (Y, X) and write them numbered to out (device memory). Ids continue
-// from *rowBase (rows written by earlier chunks); with offsetOut the rows also land at out + *rowBase rows.
-__global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double* out, const unsigned long long* rowBase,
+// from *rowBase (rows written by earlier chunks); with offsetOut the rows also land at out + *rowBase rows. The last CTA
+// to finish adds the chunk's rows to *rowBase.
+__global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double* out, unsigned long long* rowBase,
                                                             int offsetOut, unsigned long long planeBase, uint32_t capScratch)
 {
 	extern __shared__ __align__(16) unsigned long long sortSmem[];
@@ -80,7 +84,19 @@ __global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double*
 	const int f = blockIdx.x;
 	const uint32_t base = ws.frameOutBase[f];
 	const uint32_t n = ws.frameOutBase[f + 1] - base;
-	if (n == 0) { return; }
+	// every CTA has read *rowBase when the last one is counted
+	const unsigned long long idBase = *rowBase;
+	auto finished = [&]() {
+		__syncthreads();
+		if (threadIdx.x == 0) {
+			__threadfence();
+			if (atomicAdd(&ws.cnt->sorted, 1u) + 1u == gridDim.x) { *rowBase = idBase + ws.frameOutBase[ws.g.B]; }
+		}
+	};
+	if (n == 0) {
+		finished();
+		return;
+	}
 	uint32_t len = 1;
 	while (len < n) { len <<= 1; }
 	const double* __restrict__ rows = ws.rows + static_cast<long long>(base) * kCols;
@@ -91,7 +107,10 @@ __global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double*
 	else {
 		// global scratch of this frame: 2 * len keys from 4 * base and len indices from 2 * base (len < 2 n, so frames
 		// never overlap; the key scratch holds 4 * capRows and the index scratch 2 * capRows entries)
-		if (4ull * base + 2ull * len > 4ull * capScratch) { return; }
+		if (4ull * base + 2ull * len > 4ull * capScratch) {
+			finished();
+			return;
+		}
 		ky = reinterpret_cast<unsigned long long*>(ws.sortKey) + 4ull * base;
 		kx = ky + len;
 		id = ws.sortIdx + 2ull * base;
@@ -121,7 +140,6 @@ __global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double*
 	__syncthreads();
 	if (smem) { Bitonic<true>(ky, kx, id, len); }
 	else { Bitonic<false>(ky, kx, id, len); }
-	const unsigned long long idBase = *rowBase;
 	double* __restrict__ dst = out + (offsetOut ? static_cast<long long>(idBase) * kCols : 0ll) + static_cast<long long>(base) * kCols;
 	// numbered rows in sorted order, element by element (consecutive threads: consecutive columns of a row, then the
 	// next row), four elements per thread and pass with their loads issued first
@@ -147,21 +165,17 @@ __global__ void __launch_bounds__(kSortThreads) SortFrames(Workspace ws, double*
 			}
 		}
 	}
-}
-
-// After SortFrames: the chunk's rows join the running count.
-__global__ void AdvanceRowBase(Workspace ws, unsigned long long* rowBase)
-{
-	*rowBase += ws.frameOutBase[ws.g.B];
+	finished();
 }
 
 }  // namespace
 
 bool LaunchBuildCandidates(const Workspace& ws, cudaStream_t st)
 {
-	BuildCandidates<<<148 * 4, 256, 0, st>>>(ws);
+	const int blocks = static_cast<int>(std::min<uint32_t>(148 * 4, (ws.capRows + 255) / 256));
+	const bool ok = LaunchChained(BuildCandidates, blocks, 256, 0, st, ws);
 	CountLaunch();
-	return PTB_LAUNCHED();
+	return ok;
 }
 
 // out: device destination of the rows. rowBase: device count of the rows written by earlier chunks (Ids continue
@@ -173,8 +187,7 @@ bool LaunchSortFrames(const Workspace& ws, double* out, unsigned long long* rowB
 	                                                             static_cast<int>(kSortSmemBytes)));
 	if (!configured) { return false; }
 	SortFrames<<<ws.g.B, kSortThreads, kSortSmemBytes, st>>>(ws, out, rowBase, offsetOut ? 1 : 0, planeBase, ws.capRows);
-	AdvanceRowBase<<<1, 1, 0, st>>>(ws, rowBase);
-	CountLaunch(2);
+	CountLaunch();
 	return PTB_LAUNCHED();
 }
 

@@ -73,6 +73,49 @@ cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st);
 #define PTB_CUDA(call) ::ptb::CheckCuda((call), #call, __FILE__, __LINE__)
 #define PTB_LAUNCHED() ::ptb::CheckCuda(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
 
+// ---- Chained launches: a kernel launched with LaunchChained may be set up on the device while its predecessor in the
+// stream still runs (programmatic dependent launch; in a captured graph a programmatic edge). It begins with
+// PTB_AFTER_PREVIOUS(), which lets its own successor be set up and then waits for its predecessor and its writes (the
+// predecessor's end, so everything before it too); nothing before it touches memory. A chunk's segmentation is a chain
+// of some 30 short kernels whose launch gaps are as long as they are. One 256 x 256 frame on the device without a fit:
+// 45 kernels launched one after the other at full grids 156 us; 30 kernels at grids of the chunk's size 135 us, chained
+// 133 us, with the successor set up early 123 us.
+#if defined(__CUDA_ARCH__)
+#define PTB_AFTER_PREVIOUS() asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory")
+#else
+#define PTB_AFTER_PREVIOUS()
+#endif
+
+#if defined(__CUDACC__)
+template <typename... P, typename... A>
+bool LaunchChained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return PTB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+#endif
+
+// ---- Prefix sums (scan.cu): an array of n entries (*nptr, or nconst when nptr is null; cap bounds it) replaced by its
+// exclusive sums, data[n] and *total (may be null) by the total.
+struct ScanJob {
+	uint32_t* data;
+	const uint32_t* nptr;
+	uint32_t nconst, cap;
+	uint32_t* total;
+};
+constexpr int kMaxScans = 3;
+size_t ScanStateWords(uint32_t cap);
+bool ExclusiveScans(const ScanJob* jobs, int count, unsigned long long* state, uint32_t* fault, cudaStream_t st);
+
 // ---- Device counters of one chunk (one struct in device memory, read back once per chunk).
 struct Counters {
 	uint32_t ndom;      // domain pixels appended to dom[]
@@ -95,6 +138,7 @@ struct Counters {
 	uint32_t fault;        // a kernel's bounded wait ran out (its results are void; the call fails)
 	uint32_t boxNext;      // work queue of the shared-memory group floods: next multi-label group to take
 	uint32_t nunion;       // domain pixels that join two union-find trees (listed in lab for the union pass)
+	uint32_t sorted;       // frames ordered by SortFrames
 };
 
 // Why a frame is flooded again frame-wide (diagnostics, counted per frame by the first reason).
@@ -261,9 +305,12 @@ struct Workspace {
 	uint32_t* sortIdx;     // scratch for the per-frame sort
 	double* sortKey;
 	uint8_t* fitFlag;      // FP32 fits that need an FP64 re-run
-	// scan scratch
-	uint32_t* scanBlock;   // block sums
+	uint32_t* scanBlock;  // block sums of prefix sums run apart from the chunk's own (the CPU emulation)
+	// zeroed together for each chunk, one after the other (zeroBytes from cnt on): the counters, the prefix sums' states
+	// (rows, the three group arrays, regions), the per-frame arrays frameDom .. frameReflood and the root-seed bitmask
 	Counters* cnt;
+	unsigned long long* scanState;
+	size_t zeroBytes;
 };
 
 }  // namespace ptb

@@ -36,17 +36,16 @@
 // needs every pixel of the flood to be joined to a seed by a path that never falls below it, which holds for the
 // first flood (every local maximum is a seed) but not for the second flood of a basin fusion (one seed per basin):
 // there a pair failing the first test routes the frame directly.
+#include <algorithm>
+
 #include "pt_common.cuh"
 
 namespace ptb {
 
-bool ExclusiveScan(uint32_t* data, const uint32_t* nptr, uint32_t nconst, uint32_t cap, uint32_t* blockSums,
-                   uint32_t* totalOut, cudaStream_t st);
-
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kGrid = 148 * 8;  // grid-stride kernels over device-side counts: 8 CTAs per SM
+constexpr int kGrid = 148 * 8;  // grid-stride kernels over device-side counts: at most 8 CTAs per SM (GridOf)
 
 struct Pix {
 	int f, y, x;
@@ -184,6 +183,7 @@ __device__ __forceinline__ void EarlierNeighbours(const Workspace& ws, uint32_t 
 // before the seed labels and the group scatter have written every domain pixel's label.
 __global__ void CclInit(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->ndom, ws.capDom);
 	const int lane = threadIdx.x & 31;
 	PTB_WARP_LOOP(k, n)
@@ -210,6 +210,7 @@ __global__ void CclInit(Workspace ws)
 // The second union of the listed pixels (at most one per domain pixel, so the list fits lab).
 __global__ void CclUnion(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = ws.cnt->nunion;
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		const uint32_t p = ws.lab[k];
@@ -224,6 +225,7 @@ __global__ void CclUnion(Workspace ws)
 // serialises at the L2).
 __global__ void __launch_bounds__(kThreads) CompEnumerate(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ uint32_t warpBase[kThreads / 32 + 1];
 	const uint32_t n = min(ws.cnt->ndom, ws.capDom);
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(kThreads) CompEnumerate(Workspace ws)
 
 __global__ void CompCount(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->ndom, ws.capDom);
 	PTB_WARP_LOOP(k, n)
 	{
@@ -275,6 +278,7 @@ __global__ void CompCount(Workspace ws)
 // Seed parents (Segmentation2D.cpp:309-327): first seed among (y-1,x-1), (y-1,x), (y-1,x+1), (y,x-1); none = root.
 __global__ void SeedParent(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->nseed, ws.capSeed);
 	const Geometry& geo = ws.g;
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
@@ -298,6 +302,7 @@ __global__ void SeedParent(Workspace ws)
 
 __global__ void RowCount(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const Geometry& geo = ws.g;
 	const long long rows = static_cast<long long>(geo.B) * geo.H;
 	for (long long r = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; r < rows; r += gridDim.x * static_cast<long long>(blockDim.x)) {
@@ -333,6 +338,7 @@ __device__ __forceinline__ uint32_t RegionOfRoot(const Workspace& ws, uint32_t r
 
 __global__ void SeedLabel(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->nseed, ws.capSeed);
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		const uint32_t s = ws.seeds[k];
@@ -357,6 +363,7 @@ __global__ void SeedLabel(Workspace ws)
 // Groups (fast mode): components with two or more regions. Sizes go to the offset arrays, scanned next.
 __global__ void GroupEnumerate(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->ncomp, ws.capComp);
 	PTB_WARP_LOOP(c, n)
 	{
@@ -377,6 +384,7 @@ __global__ void GroupEnumerate(Workspace ws)
 // Groups (strict mode): one per frame; sizes by atomics.
 __global__ void GroupSizesStrict(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t nd = min(ws.cnt->ndom, ws.capDom);
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nd; k += gridDim.x * blockDim.x) {
 		atomicAdd(ws.gOff + Decompose(ws.dom[k], ws.g).f, 1u);
@@ -397,6 +405,7 @@ constexpr int kRedoThreads = 1024;
 
 __global__ void __launch_bounds__(kRedoThreads) RedoOffsets(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ uint32_t warpSum[3][kRedoThreads / 32];
 	__shared__ uint32_t carry[3];
 	if (ws.cnt->nroute == 0) { return; }
@@ -466,6 +475,7 @@ __device__ __forceinline__ int GroupOf(const Workspace& ws, uint32_t p, int stri
 // (their seeds get their labels back, since a fusion may have cleared them; nothing to do when no frame is routed).
 __global__ void GroupScatter(Workspace ws, int strict)
 {
+	PTB_AFTER_PREVIOUS();
 	if (strict == 2 && ws.cnt->nroute == 0) { return; }
 	const uint32_t nd = min(ws.cnt->ndom, ws.capDom);
 	const int lane = threadIdx.x & 31;
@@ -830,6 +840,7 @@ __device__ void FloodGroupGlobal(const Workspace& ws, const uint32_t* seedList, 
 // their per-component floods (routed: nothing to do when no frame did).
 __global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32_t nGroupsStrict, int routed)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ FloodSmem sm;
 	if (routed && ws.cnt->nroute == 0) { return; }
 	const uint32_t n = nGroupsStrict ? nGroupsStrict : ws.cnt->nmulti;
@@ -849,6 +860,7 @@ __global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32
 // rank: pairs failing the first exactness test are kept for the rank test (else they route the frame directly).
 __global__ void __launch_bounds__(kBoxWarps * 32) GroupFloodBox(Workspace ws, int rank)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ BoxSmem boxes[kBoxWarps];
 	BoxSmem& sm = boxes[threadIdx.x / 32];
 	const int lane = threadIdx.x & 31;
@@ -956,6 +968,7 @@ __global__ void __launch_bounds__(kBoxWarps * 32) GroupFloodBox(Workspace ws, in
 // (strict mode) or only the frames flooded again frame-wide (routed).
 __global__ void __launch_bounds__(kFloodThreads) GroupFuse(Workspace ws, uint32_t nGroupsStrict, double ratio, int routed)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ FloodSmem sm;
 	if (routed && ws.cnt->nroute == 0) { return; }
 	const uint32_t n = nGroupsStrict ? nGroupsStrict : ws.cnt->nmulti;
@@ -1090,6 +1103,7 @@ constexpr int kPlanThreads = 1024;
 // kPairsPerFrame pairs are routed instead (and get no slot). Nothing to do without such pairs.
 __global__ void __launch_bounds__(kPlanThreads) SuspectPlan(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ uint32_t warpSum[kPlanThreads / 32];
 	__shared__ uint32_t carry;
 	__shared__ uint32_t slotCount[kRankSlots], slotCur[kRankSlots];
@@ -1183,6 +1197,7 @@ __device__ __forceinline__ void PairLevels(const Workspace& ws, const uint4& r, 
 // lanes of a warp holding pixels of one slot compare them with each of the slot's pairs and add the ballot counts.
 __global__ void SuspectCount(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	if (ws.cnt->nsuspect == 0) { return; }
 	const uint32_t n = min(ws.cnt->ndom, ws.capDom);
 	const int lane = threadIdx.x & 31;
@@ -1252,6 +1267,7 @@ __device__ __forceinline__ void FailRankTest(const Workspace& ws, int f, int ref
 // estimated frame-wide aging (no basin fusion follows); else they are routed to the frame-wide flood.
 __global__ void SuspectCheck(Workspace ws, int reflood)
 {
+	PTB_AFTER_PREVIOUS();
 	if (ws.cnt->nsuspect == 0) { return; }
 	const uint32_t nrec = min(ws.cnt->nsuspect, ws.capSuspect);
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nrec; i += gridDim.x * blockDim.x) {
@@ -1278,6 +1294,7 @@ __global__ void SuspectCheck(Workspace ws, int reflood)
 // Step 1 (one CTA): slots for the frames marked by the rank test, in frame order; the others are routed.
 __global__ void __launch_bounds__(kPlanThreads) RefloodPlan(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ uint32_t next;
 	if (ws.cnt->nreflood == 0) { return; }
 	if (threadIdx.x == 0) { next = 0; }
@@ -1323,6 +1340,7 @@ __device__ __forceinline__ bool Poppable(const Workspace& ws, uint32_t p)
 // multi-label groups, which the next steps walk instead of every group of the chunk.
 __global__ void RefloodGather(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	if (ws.cnt->nreflood == 0) { return; }
 	const int lane = threadIdx.x & 31;
 	const uint32_t N = static_cast<uint32_t>(ws.g.N);
@@ -1383,6 +1401,7 @@ constexpr size_t kRfBucketSmem = kRefloodBuckets * sizeof(uint32_t);
 // smallest that fits the value range in kRefloodBuckets buckets), bucket offsets by a counting pass in shared memory.
 __global__ void __launch_bounds__(kRfBucketThreads) RefloodBucket(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	extern __shared__ uint32_t hist[];  // [kRefloodBuckets]: counts, then cursors
 	__shared__ uint32_t red[2][kRfBucketThreads / 32];
 	__shared__ uint32_t carry;
@@ -1491,6 +1510,7 @@ __device__ __forceinline__ uint32_t FrameDelta(const Workspace& ws, int f)
 // #{W1 > W1(p)} and its upper bound B(p) = #{W1 >= W1(p) - delta}.
 __global__ void RefloodCounts(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	if (ws.cnt->nreflood == 0) { return; }
 	const uint32_t nList = ws.cnt->nrfgroup;
 	const int lane = threadIdx.x & 31;
@@ -1658,6 +1678,7 @@ __device__ bool RefloodGroupGlobal(const Workspace& ws, RfBoxSmem& sm, uint32_t 
 // fails the first test; a failing frame is routed to the frame-wide flood.
 __global__ void __launch_bounds__(kRfWarps * 32) RefloodBox(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	__shared__ RfBoxSmem boxes[kRfWarps];
 	if (ws.cnt->nreflood == 0) { return; }
 	RfBoxSmem& sm = boxes[threadIdx.x / 32];
@@ -1802,6 +1823,7 @@ __global__ void __launch_bounds__(kRfWarps * 32) RefloodBox(Workspace ws)
 // there is one set of atomics per run instead of per pixel (integer sums: the order does not matter).
 __global__ void RegionStats(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = min(ws.cnt->ndom, ws.capDom);
 	const Geometry& geo = ws.g;
 	PTB_WARP_LOOP(k, n)
@@ -1835,6 +1857,7 @@ __global__ void RegionStats(Workspace ws)
 
 __global__ void CandidateFlags(Workspace ws)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = ws.cnt->nregion;
 	for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
 		ws.regCand[r] = static_cast<double>(ws.regCount[r]) > kVolumeMin ? 1u : 0u;  // FilterData, :88-141
@@ -1844,6 +1867,7 @@ __global__ void CandidateFlags(Workspace ws)
 // Per frame: candidate base, kept count (capacity truncation in label order, Fitting.cpp:44-58) and output base.
 __global__ void FrameCandidates(Workspace ws, uint32_t maxPoints)
 {
+	PTB_AFTER_PREVIOUS();
 	const int B = ws.g.B;
 	for (int f = blockIdx.x * blockDim.x + threadIdx.x; f <= B; f += gridDim.x * blockDim.x) {
 		const uint32_t rb = ws.rowcnt[static_cast<long long>(f) * ws.g.H];
@@ -1854,6 +1878,7 @@ __global__ void FrameCandidates(Workspace ws, uint32_t maxPoints)
 
 __global__ void FrameKeep(Workspace ws, uint32_t maxPoints)
 {
+	PTB_AFTER_PREVIOUS();
 	const int B = ws.g.B;
 	for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < B; f += gridDim.x * blockDim.x) {
 		const uint32_t c = ws.frameCandBase[f + 1] - ws.frameCandBase[f];
@@ -1862,8 +1887,54 @@ __global__ void FrameKeep(Workspace ws, uint32_t maxPoints)
 	}
 }
 
+// FrameCandidates, FrameKeep and the prefix sum of the kept counts in one CTA, for chunks of few frames.
+constexpr int kOffsetThreads = 1024;
+constexpr int kOffsetFrames = 4096;
+
+__global__ void __launch_bounds__(kOffsetThreads) FrameOffsets(Workspace ws, uint32_t maxPoints)
+{
+	PTB_AFTER_PREVIOUS();
+	__shared__ uint32_t warpSum[kOffsetThreads / 32];
+	const int B = ws.g.B, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	uint32_t carry = 0;
+	for (int base = 0; base <= B; base += kOffsetThreads) {
+		const int f = base + static_cast<int>(threadIdx.x);
+		uint32_t keep = 0;
+		if (f <= B) {
+			const uint32_t rb = ws.rowcnt[static_cast<long long>(f) * ws.g.H], cb = ws.regCand[rb];
+			ws.frameRegBase[f] = rb;
+			ws.frameCandBase[f] = cb;
+			if (f < B) {
+				const uint32_t c = ws.regCand[ws.rowcnt[static_cast<long long>(f + 1) * ws.g.H]] - cb;
+				keep = min(c, maxPoints);
+				ws.frameKeep[f] = keep;
+				if (c > maxPoints) { atomicExch(&ws.cnt->truncated, 1u); }
+			}
+		}
+		uint32_t x = keep;
+		#pragma unroll
+		for (int d = 1; d < 32; d <<= 1) {
+			const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+			if (lane >= d) { x += y; }
+		}
+		if (lane == 31) { warpSum[warp] = x; }
+		__syncthreads();
+		uint32_t before = 0, total = 0;
+		for (int w = 0; w < kOffsetThreads / 32; ++w) {
+			const uint32_t v = warpSum[w];
+			before += w < warp ? v : 0u;
+			total += v;
+		}
+		if (f <= B) { ws.frameOutBase[f] = carry + before + x - keep; }
+		carry += total;
+		__syncthreads();
+	}
+	if (threadIdx.x == 0) { ws.cnt->nfit = carry; }
+}
+
 __global__ void CandidateEmit(Workspace ws, uint32_t maxPoints)
 {
+	PTB_AFTER_PREVIOUS();
 	const uint32_t n = ws.cnt->nregion;
 	for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
 		if (!(static_cast<double>(ws.regCount[r]) > kVolumeMin)) { continue; }
@@ -1877,115 +1948,106 @@ __global__ void CandidateEmit(Workspace ws, uint32_t maxPoints)
 	}
 }
 
+// CTAs of the grid-stride kernels for a chunk of P pixels: one per 2048 pixels (the lists hold a few per cent of them),
+// at least 16, at most kGrid. A full grid takes about 2 us to start and end, most of a short kernel's time.
+int GridOf(const Workspace& ws)
+{
+	return static_cast<int>(std::min<long long>(kGrid, std::max<long long>(16, (ws.g.P + 2047) / 2048)));
+}
+
 }  // namespace
 
 // Runs the whole segmentation of a chunk after detection. `strict` selects frame-wide floods.
 bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPoints, cudaStream_t st)
 {
 	const Geometry& g = ws.g;
+	const int grid = GridOf(ws);
 	bool ok = true;
-	CclInit<<<kGrid, kThreads, 0, st>>>(ws);
-	CclUnion<<<kGrid, kThreads, 0, st>>>(ws);
-	CompEnumerate<<<kGrid, kThreads, 0, st>>>(ws);
-	CompCount<<<kGrid, kThreads, 0, st>>>(ws);
-	SeedParent<<<kGrid, kThreads, 0, st>>>(ws);
-	RowCount<<<kGrid, kThreads, 0, st>>>(ws);
-	CountLaunch(6);
-	ok = ok && PTB_LAUNCHED();
+	auto launch = [&](auto kernel, int blocks, int threads, auto... args) {
+		ok = ok && LaunchChained(kernel, blocks, threads, 0, st, ws, args...);
+		CountLaunch();
+	};
+	// the prefix sums' states follow one another in the order of their workspace slots
 	const uint32_t rows = static_cast<uint32_t>(g.B) * static_cast<uint32_t>(g.H);
-	ok = ok && ExclusiveScan(ws.rowcnt, nullptr, rows, rows, ws.scanBlock, &ws.cnt->nregion, st);
-	SeedLabel<<<kGrid, kThreads, 0, st>>>(ws);
-	CountLaunch();
-	ok = ok && PTB_LAUNCHED();
+	unsigned long long* const rowState = ws.scanState;
+	unsigned long long* const groupState = rowState + ScanStateWords(rows);
+	unsigned long long* const regionState = groupState + 3 * ScanStateWords(ws.capComp);
+	auto scan = [&](std::initializer_list<ScanJob> jobs, unsigned long long* state) {
+		ok = ok && ExclusiveScans(jobs.begin(), static_cast<int>(jobs.size()), state, &ws.cnt->fault, st);
+	};
+	launch(CclInit, grid, kThreads);
+	launch(CclUnion, grid, kThreads);
+	launch(CompEnumerate, grid, kThreads);
+	launch(CompCount, grid, kThreads);
+	launch(SeedParent, grid, kThreads);
+	launch(RowCount, grid, kThreads);
+	scan({{ws.rowcnt, nullptr, rows, rows, &ws.cnt->nregion}}, rowState);
+	launch(SeedLabel, grid, kThreads);
 	// mode 0: per-component floods with both exactness tests; 2: with the first test only; 1: frame-wide floods
 	const int rank = strict == 0 ? 1 : 0;
 	strict = strict == 1 ? 1 : 0;
-	const uint32_t groupsStrict = strict ? static_cast<uint32_t>(g.B) : 0u;
+	const uint32_t frames = static_cast<uint32_t>(g.B);
+	const uint32_t groupsStrict = strict ? frames : 0u;
 	if (strict) {
-		PTB_CUDA(cudaMemsetAsync(ws.gOff, 0, sizeof(uint32_t) * (g.B + 1), st));
-		PTB_CUDA(cudaMemsetAsync(ws.gSeedOff, 0, sizeof(uint32_t) * (g.B + 1), st));
-		PTB_CUDA(cudaMemsetAsync(ws.gRegOff, 0, sizeof(uint32_t) * (g.B + 1), st));
-		PTB_CUDA(cudaMemsetAsync(ws.gCurPix, 0, sizeof(uint32_t) * (g.B + 1), st));
-		PTB_CUDA(cudaMemsetAsync(ws.gCurSeed, 0, sizeof(uint32_t) * (g.B + 1), st));
-		PTB_CUDA(cudaMemsetAsync(ws.gCurReg, 0, sizeof(uint32_t) * (g.B + 1), st));
-		GroupSizesStrict<<<kGrid, kThreads, 0, st>>>(ws);
-		CountLaunch();
-		ok = ok && PTB_LAUNCHED();
-		ok = ok && ExclusiveScan(ws.gOff, nullptr, groupsStrict, groupsStrict, ws.scanBlock, nullptr, st);
-		ok = ok && ExclusiveScan(ws.gSeedOff, nullptr, groupsStrict, groupsStrict, ws.scanBlock, nullptr, st);
-		ok = ok && ExclusiveScan(ws.gRegOff, nullptr, groupsStrict, groupsStrict, ws.scanBlock, nullptr, st);
+		for (uint32_t* list : {ws.gOff, ws.gSeedOff, ws.gRegOff, ws.gCurPix, ws.gCurSeed, ws.gCurReg}) {
+			ok = ok && PTB_CUDA(cudaMemsetAsync(list, 0, sizeof(uint32_t) * (g.B + 1), st));
+		}
+		launch(GroupSizesStrict, grid, kThreads);
+		scan({{ws.gOff, nullptr, frames, ws.capComp, nullptr}, {ws.gSeedOff, nullptr, frames, ws.capComp, nullptr},
+		      {ws.gRegOff, nullptr, frames, ws.capComp, nullptr}}, groupState);
 	}
 	else {
-		GroupEnumerate<<<kGrid, kThreads, 0, st>>>(ws);
-		CountLaunch();
-		ok = ok && PTB_LAUNCHED();
-		ok = ok && ExclusiveScan(ws.gOff, &ws.cnt->nmulti, 0, ws.capComp, ws.scanBlock, nullptr, st);
-		ok = ok && ExclusiveScan(ws.gSeedOff, &ws.cnt->nmulti, 0, ws.capComp, ws.scanBlock, nullptr, st);
-		ok = ok && ExclusiveScan(ws.gRegOff, &ws.cnt->nmulti, 0, ws.capComp, ws.scanBlock, nullptr, st);
+		launch(GroupEnumerate, grid, kThreads);
+		scan({{ws.gOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr}, {ws.gSeedOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr},
+		      {ws.gRegOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr}}, groupState);
 	}
-	GroupScatter<<<kGrid, kThreads, 0, st>>>(ws, strict ? 1 : 0);
+	launch(GroupScatter, grid, kThreads, strict ? 1 : 0);
 	if (strict) {  // frame-wide groups: one thread per group, small CTAs so that many SMs share the frames
-		GroupFlood<<<kGrid * 2, kFloodThreads, 0, st>>>(ws, groupsStrict, 0);
+		launch(GroupFlood, grid * 2, kFloodThreads, groupsStrict, 0);
 	}
 	else {  // one warp per group, staged in shared memory
-		GroupFloodBox<<<kGrid, kBoxWarps * 32, 0, st>>>(ws, rank);
+		launch(GroupFloodBox, grid, kBoxWarps * 32, rank);
 	}
-	CountLaunch(2);
-	ok = ok && PTB_LAUNCHED();
 	const bool fuse = static_cast<int>(ratio) > 0;  // WatershedIntelligent, Segmentation2D.cpp:77-85
-	if (fuse) {
-		GroupFuse<<<kGrid * 2, kFloodThreads, 0, st>>>(ws, groupsStrict, ratio, 0);
-		CountLaunch();
-		ok = ok && PTB_LAUNCHED();
-	}
+	if (fuse) { launch(GroupFuse, grid * 2, kFloodThreads, groupsStrict, ratio, 0); }
 	if (!strict) {
 		// boundary pairs that failed the first exactness test: the rank test of their frames (each kernel returns at
 		// once when no pair failed)
 		if (rank) {
-			SuspectPlan<<<1, kPlanThreads, 0, st>>>(ws);
-			SuspectCount<<<kGrid, kThreads, 0, st>>>(ws);
+			launch(SuspectPlan, 1, kPlanThreads);
+			launch(SuspectCount, grid, kThreads);
 			// frames failing the rank test: flooded again with estimated frame-wide aging (not after a basin fusion,
 			// which used the first flood's labels)
-			SuspectCheck<<<64, kThreads, 0, st>>>(ws, fuse ? 0 : 1);
-			RefloodPlan<<<1, kPlanThreads, 0, st>>>(ws);
-			RefloodGather<<<kGrid, kThreads, 0, st>>>(ws);
+			launch(SuspectCheck, std::min(grid, 64), kThreads, fuse ? 0 : 1);
+			launch(RefloodPlan, 1, kPlanThreads);
+			launch(RefloodGather, grid, kThreads);
 			static const bool bucketSmem = PTB_CUDA(cudaFuncSetAttribute(RefloodBucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
 			                                                             static_cast<int>(kRfBucketSmem)));
-			ok = ok && bucketSmem;
-			RefloodBucket<<<kRefloodSlots * 2, kRfBucketThreads, kRfBucketSmem, st>>>(ws);
-			RefloodCounts<<<kGrid, kThreads, 0, st>>>(ws);
-			RefloodBox<<<kGrid, kRfWarps * 32, 0, st>>>(ws);
-			CountLaunch(8);
-			ok = ok && PTB_LAUNCHED();
+			ok = ok && bucketSmem && LaunchChained(RefloodBucket, kRefloodSlots * 2, kRfBucketThreads, kRfBucketSmem, st, ws);
+			CountLaunch();
+			launch(RefloodCounts, grid, kThreads);
+			launch(RefloodBox, grid, kRfWarps * 32);
 		}
 		// frames whose per-component floods failed the exactness tests: flooded again as one unit with the frame-global
 		// pop counter (each kernel returns at once when no frame was routed)
-		const uint32_t frames = static_cast<uint32_t>(g.B);
-		RedoOffsets<<<1, kRedoThreads, 0, st>>>(ws);
-		GroupScatter<<<kGrid, kThreads, 0, st>>>(ws, 2);
-		GroupFlood<<<kGrid * 2, kFloodThreads, 0, st>>>(ws, frames, 1);
-		CountLaunch(3);
-		if (fuse) {
-			GroupFuse<<<kGrid * 2, kFloodThreads, 0, st>>>(ws, frames, ratio, 1);
-			CountLaunch();
-		}
-		ok = ok && PTB_LAUNCHED();
+		launch(RedoOffsets, 1, kRedoThreads);
+		launch(GroupScatter, grid, kThreads, 2);
+		launch(GroupFlood, grid * 2, kFloodThreads, frames, 1);
+		if (fuse) { launch(GroupFuse, grid * 2, kFloodThreads, frames, ratio, 1); }
 	}
-	RegionStats<<<kGrid, kThreads, 0, st>>>(ws);
-	CandidateFlags<<<kGrid, kThreads, 0, st>>>(ws);
-	CountLaunch(2);
-	ok = ok && PTB_LAUNCHED();
-	ok = ok && ExclusiveScan(ws.regCand, &ws.cnt->nregion, 0, ws.capRegion, ws.scanBlock, &ws.cnt->ncand, st);
-	FrameCandidates<<<(g.B + 256) / 256, 256, 0, st>>>(ws, maxPoints);
-	FrameKeep<<<(g.B + 255) / 256, 256, 0, st>>>(ws, maxPoints);
-	CountLaunch(2);
-	ok = ok && PTB_LAUNCHED();
-	PTB_CUDA(cudaMemcpyAsync(ws.frameOutBase, ws.frameKeep, sizeof(uint32_t) * g.B, cudaMemcpyDeviceToDevice, st));
-	ok = ok && ExclusiveScan(ws.frameOutBase, nullptr, static_cast<uint32_t>(g.B), static_cast<uint32_t>(g.B), ws.scanBlock,
-	                         &ws.cnt->nfit, st);
-	CandidateEmit<<<kGrid, kThreads, 0, st>>>(ws, maxPoints);
-	CountLaunch();
-	ok = ok && PTB_LAUNCHED();
+	launch(RegionStats, grid, kThreads);
+	launch(CandidateFlags, grid, kThreads);
+	scan({{ws.regCand, &ws.cnt->nregion, 0, ws.capRegion, &ws.cnt->ncand}}, regionState);
+	if (g.B <= kOffsetFrames) { launch(FrameOffsets, 1, kOffsetThreads, maxPoints); }
+	else {
+		launch(FrameCandidates, (g.B + 256) / 256, 256, maxPoints);
+		launch(FrameKeep, (g.B + 255) / 256, 256, maxPoints);
+		ok = ok && PTB_CUDA(cudaMemcpyAsync(ws.frameOutBase, ws.frameKeep, sizeof(uint32_t) * g.B, cudaMemcpyDeviceToDevice, st));
+		// the rows' state is free again
+		ok = ok && PTB_CUDA(cudaMemsetAsync(rowState, 0, ScanStateWords(frames) * sizeof(unsigned long long), st));
+		scan({{ws.frameOutBase, nullptr, frames, frames, &ws.cnt->nfit}}, rowState);
+	}
+	launch(CandidateEmit, grid, kThreads, maxPoints);
 	return ok;
 }
 

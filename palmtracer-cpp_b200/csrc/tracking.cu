@@ -29,9 +29,6 @@
 
 namespace ptb {
 
-bool ExclusiveScan(uint32_t* data, const uint32_t* nptr, uint32_t nconst, uint32_t cap, uint32_t* blockSums,
-                   uint32_t* totalOut, cudaStream_t st);
-
 namespace {
 
 constexpr uint32_t kNoLink = 0xffffffffu;
@@ -433,21 +430,28 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 	}
 	const uint32_t P = static_cast<uint32_t>(span + 1);
 	const uint64_t minPlane = hostMinMax[0];
-	uint32_t *begin = nullptr, *cursor = nullptr, *scanScratch = nullptr;
+	uint32_t *begin = nullptr, *cursor = nullptr, *fault = nullptr;
+	unsigned long long* scanState = nullptr;  // planes, pairs, chain heads, one after the other
 	unsigned long long *pk1 = nullptr, *pk2 = nullptr, *s1 = nullptr, *s2 = nullptr;
 	double2* xy = nullptr;
 	uint32_t* rel = nullptr;
 	unsigned long long *xk1 = nullptr, *xk2 = nullptr;
-	const uint32_t scanCap = std::max(n, P) + 2;
-	ok = alloc(begin, P + 2) && alloc(cursor, P) && alloc(scanScratch, scanCap / 4096 + 2) && alloc(pk1, n) && alloc(pk2, n) &&
+	const size_t planeWords = ScanStateWords(P + 1), pointWords = ScanStateWords(n + 1), scanWords = planeWords + 2 * pointWords;
+	auto scan = [&](uint32_t* data, uint32_t count, size_t at) {
+		const ScanJob job{data, nullptr, count, count, nullptr};
+		return ExclusiveScans(&job, 1, scanState + at, fault, st);
+	};
+	ok = alloc(begin, P + 2) && alloc(cursor, P) && alloc(scanState, scanWords + 1) && alloc(pk1, n) && alloc(pk2, n) &&
 	     alloc(s1, 2ull * n) && alloc(s2, 2ull * n) && alloc(xy, n) && alloc(rel, n) && alloc(xk1, n) && alloc(xk2, n);
 	ok = ok && PTB_CUDA(cudaMemsetAsync(begin, 0, sizeof(uint32_t) * (P + 2), st)) &&
-	     PTB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * P, st));
+	     PTB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(uint32_t) * P, st)) &&
+	     PTB_CUDA(cudaMemsetAsync(scanState, 0, sizeof(unsigned long long) * (scanWords + 1), st));
+	fault = reinterpret_cast<uint32_t*>(scanState + scanWords);
 	if (ok) {
 		// (Plane, Id) order: counting sort by plane, then (Id, input index) inside each plane
 		PlaneCount<<<G, kTrackThreads, 0, st>>>(plane, n, minPlane, begin);
 		CountLaunch();
-		ok = PTB_LAUNCHED() && ExclusiveScan(begin, nullptr, P + 1, P + 1, scanScratch, nullptr, st);
+		ok = PTB_LAUNCHED() && scan(begin, P + 1, 0);
 	}
 	if (ok) {
 		PlaneScatter<<<G, kTrackThreads, 0, st>>>(plane, id, n, minPlane, begin, cursor, pk1, pk2);
@@ -483,7 +487,7 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 	uint32_t *off = nullptr, *next = nullptr, *prev = nullptr, *head = nullptr, *root = nullptr;
 	unsigned long long *ck1 = nullptr, *ck2 = nullptr, *c1 = nullptr, *c2 = nullptr, *tgtD2 = nullptr;
 	uint32_t *tgtSrc = nullptr, *pending = nullptr;
-	ok = ok && ExclusiveScan(pairBegin, nullptr, n, n + 1, scanScratch, nullptr, st);
+	ok = ok && scan(pairBegin, n, planeWords);
 	ok = ok && alloc(ck1, pairs) && alloc(ck2, pairs) && alloc(c1, 2 * pairs) && alloc(c2, 2 * pairs) && alloc(off, P + 1) &&
 	     alloc(next, n) && alloc(prev, n) && alloc(head, n + 2) && alloc(root, n) && alloc(tgtD2, n) && alloc(tgtSrc, n) && alloc(pending, P);
 	if (ok && pairs > 0) {
@@ -508,7 +512,7 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 	if (ok) {
 		HeadFlags<<<G, kTrackThreads, 0, st>>>(prev, n, head, root);
 		CountLaunch();
-		ok = PTB_LAUNCHED() && ExclusiveScan(head, nullptr, n, n + 1, scanScratch, nullptr, st);
+		ok = PTB_LAUNCHED() && scan(head, n, planeWords + pointWords);
 	}
 	// a chain has at most one point per plane
 	int rounds = 1;
@@ -522,6 +526,12 @@ bool TrackDevice(const double* dIn, uint64_t* dOut, uint64_t nPoints, double max
 		TrackOutput<<<G, kTrackThreads, 0, st>>>(pk1, root, head, n, dOut);
 		CountLaunch();
 		ok = PTB_LAUNCHED();
+	}
+	uint32_t late = 0;
+	ok = ok && PTB_CUDA(cudaMemcpyAsync(&late, fault, sizeof(late), cudaMemcpyDeviceToHost, st)) && PTB_CUDA(cudaStreamSynchronize(st));
+	if (ok && late != 0) {
+		SetError("Tracking: a prefix sum's bounded wait for a predecessor ran out");
+		ok = false;
 	}
 	release();
 	return ok;

@@ -139,6 +139,8 @@ struct Counters {
 	uint32_t boxNext;      // work queue of the shared-memory group floods: next multi-label group to take
 	uint32_t nunion;       // domain pixels that join two union-find trees (listed in lab for the union pass)
 	uint32_t sorted;       // frames ordered by SortFrames
+	uint32_t fuseNext;     // work queue of the shared-memory basin fusions: next multi-label group to take
+	uint32_t nfuse;        // groups too large for them (listed in rfGroups, which the re-flood does not use after a fusion)
 };
 
 // Why a frame is flooded again frame-wide (diagnostics, counted per frame by the first reason).

@@ -150,15 +150,16 @@ size_t ScanStateWords(uint32_t cap) { return static_cast<size_t>(Tiles(cap)) + 2
 bool ExclusiveScans(const ScanJob* jobs, int count, unsigned long long* state, uint32_t* fault, cudaStream_t st)
 {
 	Scans s{};
-	uint32_t tiles = 1;
+	uint32_t blocks = 1;
 	for (int k = 0; k < count; ++k) {
 		s.job[k] = jobs[k];
 		s.state[k] = state;
 		state += ScanStateWords(jobs[k].cap);
-		tiles = std::max(tiles, Tiles(jobs[k].cap));
+		// a count known only on the device is a few per cent of its capacity: a CTA per 16 tiles of that
+		blocks = std::max(blocks, jobs[k].nptr ? Tiles(jobs[k].cap) / 16 : Tiles(jobs[k].nconst));
 	}
 	s.fault = fault;
-	const bool ok = LaunchChained(ScanKernel, dim3(std::min<uint32_t>(tiles, 148u), count), kScanThreads, 0, st, s);
+	const bool ok = LaunchChained(ScanKernel, dim3(std::min<uint32_t>(blocks, 148u), count), kScanThreads, 0, st, s);
 	CountLaunch();
 	return ok;
 }

@@ -173,8 +173,8 @@ PTB_API uint64_t PTB_FittingDeviceNoAlloc(const uint16_t* d_input, const double*
  * Boundaries failing it get the rank test, whose bound comes from the counts of the frame's pixels above and below
  * the two W1 levels (the frame-wide flood pops in W1 order up to the aging term). A frame failing the rank test is
  * flooded again per component with each pop's aging set to its estimated frame-wide position, and tested again with
- * per-element bounds; only a frame failing that too (or, with basin fusion, the rank test) is flooded again as one
- * unit with the frame-global pop counter. 1 (strict): every frame is flooded as one unit.
+ * per-element bounds; only a frame failing that too (or, with basin fusion, the first test of the fused basins' flood) is
+ * flooded again as one unit with the frame-global pop counter. 1 (strict): every frame is flooded as one unit.
  * 2: as 0 with the first test only (every frame failing it is flooded again frame-wide; for comparisons).
  * Other values select 0. Returns the previous mode. */
 PTB_API int PTB_SetSegmentationMode(int mode);
@@ -184,8 +184,8 @@ PTB_API int PTB_SetSegmentationMode(int mode);
  * second exactness test) in mode 0, counts[3] frames flooded again per component with estimated frame-wide aging
  * after failing it, counts[4..10] the frames of counts[1] by the first reason they were flooded frame-wide: the list
  * of failing boundary pairs full, a pair failing the first test in mode 2, no rank-test slot left in the chunk, too
- * many failing pairs in the frame, a failed rank test after a basin fusion, no re-flood slot or too many domain
- * pixels for the re-flood, a failed re-flood test (up to n entries). */
+ * many failing pairs in the frame, always 0, no re-flood slot or too many domain pixels for the re-flood, a failed
+ * re-flood test (up to n entries). */
 PTB_API void PTB_SegmentationStats(uint64_t* counts, int n);
 
 /* Engine pool of the current device (diagnostics): counts[0] engines created, counts[1] the most engines leased at

@@ -289,11 +289,12 @@ static size_t PlanWorkspace(Workspace& ws, int H, int W, int B, uint32_t rowsCap
 	take(ws.fuNeighbour, capComp);
 	take(ws.fuBecome, capComp);
 	take(ws.fuLocked, capComp);
-	take(ws.rfVals, static_cast<size_t>(kRefloodSlots) * 2 * kRefloodCap);
-	take(ws.rfGrp, static_cast<size_t>(kRefloodSlots) * 2 * kRefloodCap);
-	take(ws.rfOff, static_cast<size_t>(kRefloodSlots) * 2 * (kRefloodBuckets + 1));
+	const size_t slots = RefloodSlots(g);
+	take(ws.rfVals, slots * 2 * kRefloodCap);
+	take(ws.rfGrp, slots * 2 * kRefloodCap);
+	take(ws.rfOff, slots * 2 * (kRefloodBuckets + 1));
 	take(ws.rfInfo, static_cast<size_t>(kRefloodSlots) * 8);
-	take(ws.rfPix, static_cast<size_t>(kRefloodSlots) * static_cast<size_t>(g.N) * kRfWords);
+	take(ws.rfPix, slots * static_cast<size_t>(g.N) * kRfWords);
 	take(ws.rfGroups, capComp);
 	take(ws.suspect, kSuspectCap);
 	take(ws.rankOrder, kSuspectCap);
@@ -436,7 +437,10 @@ int Engine::ChunkFrames(int H, int W, uint64_t planes, uint32_t maxPoints, size_
 	// bytes per frame: ~40 B per pixel of dense lists plus ~100 B per independent-set slot plus fit rows
 	const double perFrame = 48.0 * N + 100.0 * IndepBound(H, W) +
 	                        std::min<double>(maxPoints, IndepBound(H, W)) * 360.0 + 2.0 * N;
-	long long B = static_cast<long long>(static_cast<double>(budget) / perFrame);
+	// the re-flood slots hold kRfWords words per pixel of their frame, a slot per frame up to kRefloodSlots
+	const double slot = 4.0 * kRfWords * N;
+	long long B = static_cast<long long>((static_cast<double>(budget) - kRefloodSlots * slot) / perFrame);
+	if (B < static_cast<long long>(kRefloodSlots)) { B = static_cast<long long>(static_cast<double>(budget) / (perFrame + slot)); }
 	B = std::max<long long>(1, std::min<long long>(B, static_cast<long long>(planes)));
 	// global pixel indices of a chunk stay below 2^31 (the top bit tags component ids)
 	B = std::min<long long>(B, std::max<long long>(1, ((1ll << 31) - 1) / std::max<long long>(N, 1)));

@@ -41,8 +41,9 @@ constexpr uint32_t kSuspectCap = 16384u;
 constexpr uint32_t kPairsPerFrame = 512u;
 // Re-flood of the frames that fail the rank test: at most kRefloodSlots frames per chunk, each with at most
 // kRefloodCap domain pixels (their W1 values are grouped by value bucket for the rank lookups); other frames are
-// flooded frame-wide.
-constexpr uint32_t kRefloodSlots = 8u;
+// flooded frame-wide. About 1 in 100 frames of 1024 x 1024 fails: of 30 stacks of 500 frames, two had more than 8 such
+// frames in a chunk and took 290 ms instead of 10 with 8 slots.
+constexpr uint32_t kRefloodSlots = 32u;
 constexpr uint32_t kRefloodCap = 65536u;
 constexpr uint32_t kRefloodBuckets = 32768u;  // value buckets of the rank lookups
 // Words per pixel and re-flood slot of rfPix: the estimated frame-wide pop position, its bound B, and for groups
@@ -149,7 +150,7 @@ enum RouteReason : int {
 	kRouteFirstTest = 1,    // a pair failed the first test where no rank test follows (segmentation mode 2)
 	kRouteRankSlots = 2,    // more frames needed the rank test than a chunk has slots
 	kRoutePairs = 3,        // the frame had more failing pairs than the rank test takes per frame
-	kRouteRankFused = 4,    // failed the rank test after a basin fusion (no re-flood)
+	kRouteRankFused = 4,    // (none: the rank test comes before the fusion)
 	kRouteRefloodSlots = 5, // failed the rank test beyond the re-flood slots or the re-flood's domain-pixel capacity
 	kRouteRefloodTest = 6   // the re-flooded labels failed the per-element rank test
 };
@@ -247,6 +248,12 @@ struct Geometry {
 	FastDiv divN, divW;
 };
 
+// Re-flood slots of a chunk.
+__host__ __device__ __forceinline__ uint32_t RefloodSlots(const Geometry& g)
+{
+	return static_cast<uint32_t>(g.B) < kRefloodSlots ? static_cast<uint32_t>(g.B) : kRefloodSlots;
+}
+
 // Device workspace of one chunk. Dense arrays have P entries, lists have their stated capacities.
 struct Workspace {
 	Geometry g;
@@ -289,10 +296,10 @@ struct Workspace {
 	uint32_t* rankOrder; uint32_t* rankSlotOff; uint32_t* rankCount;
 	// per frame [B + 1]: nonzero where the frame failed the rank test (then its re-flood slot + 1); per slot and list
 	// (0: the W1 values of its domain pixels, 1: of the pixels its frame-wide flood pops): the values as gathered and
-	// grouped by value bucket ([kRefloodSlots][2][kRefloodCap]), the bucket offsets ([kRefloodSlots][2][buckets + 1]);
+	// grouped by value bucket ([slots][2][kRefloodCap]), the bucket offsets ([slots][2][buckets + 1]);
 	// per slot [8]: the two counts, the frame + 1, unused, and per list the lowest value and the bucket shift; per slot
 	// and pixel of the frame: the estimated frame-wide pop position and its upper bound, then the global re-flood's
-	// element value and chain minimum ([kRefloodSlots][N][kRfWords]); the
+	// element value and chain minimum ([slots][N][kRfWords]), slots = RefloodSlots(geometry); the
 	// multi-label groups of the slotted frames ([capComp])
 	uint32_t* frameReflood;
 	uint32_t* rfVals; uint32_t* rfGrp; uint32_t* rfOff; uint32_t* rfInfo; uint32_t* rfPix; uint32_t* rfGroups;

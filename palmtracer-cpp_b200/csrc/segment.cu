@@ -553,7 +553,7 @@ __device__ void SortSlice(uint32_t* a, uint32_t n)
 // equal keys come out in the same order as from the reference's std::priority_queue.
 // Entry i lives at key[i * stride], pix[i * stride]: a lane-interleaved slice of shared memory while the heap holds at
 // most `cap` entries, then (Spill) the group's own slice of global memory, sized for the whole group.
-struct Heap {
+struct HeapStore {
 	double* key;
 	uint32_t* pix;
 	uint32_t len;
@@ -561,10 +561,29 @@ struct Heap {
 	uint32_t cap;
 	double* gkey;
 	uint32_t* gpix;
-
-	__device__ __forceinline__ static bool Less(double a, double b) { return a > b; }
 	__device__ __forceinline__ double& K(uint32_t i) { return key[i * stride]; }
 	__device__ __forceinline__ uint32_t& P(uint32_t i) { return pix[i * stride]; }
+};
+
+// Entries 0 .. kFrameHeap - 1 at key and pix, the rest in the group's slice of global memory (no spill).
+constexpr uint32_t kFrameHeap = 16384u;
+struct SplitStore : HeapStore {
+	__device__ __forceinline__ double& K(uint32_t i) { return i < kFrameHeap ? key[i] : gkey[i]; }
+	__device__ __forceinline__ uint32_t& P(uint32_t i) { return i < kFrameHeap ? pix[i] : gpix[i]; }
+};
+
+template <class Store>
+struct HeapOn : Store {
+	using Store::K;
+	using Store::P;
+	using Store::cap;
+	using Store::gkey;
+	using Store::gpix;
+	using Store::key;
+	using Store::len;
+	using Store::pix;
+	using Store::stride;
+	__device__ __forceinline__ static bool Less(double a, double b) { return a > b; }
 
 	__device__ void Spill()
 	{
@@ -630,6 +649,9 @@ struct Heap {
 		return top;
 	}
 };
+
+using Heap = HeapOn<HeapStore>;
+using SplitHeap = HeapOn<SplitStore>;
 
 constexpr int kFloodThreads = 64;
 constexpr uint32_t kSmemHeap = 48;  // shared-memory heap entries per thread (12 bytes each)
@@ -937,24 +959,256 @@ template <bool kChain>
 __device__ void FloodGroupGlobal(const Workspace& ws, const uint32_t* seedList, uint32_t nSeeds, double* hk, uint32_t* hp,
                                  FloodSmem& sm)
 {
-	Heap heap{sm.key + threadIdx.x, sm.pix + threadIdx.x, 0, kFloodThreads, kSmemHeap, hk, hp};
+	Heap heap{{sm.key + threadIdx.x, sm.pix + threadIdx.x, 0, kFloodThreads, kSmemHeap, hk, hp}};
 	FloodGroup<kChain>(ws.g, GlobalView{ws}, seedList, nSeeds, heap);
 }
 
-// Frame-wide floods (groups = frames): every frame (strict mode) or only the frames that failed the exactness test of
-// their per-component floods (routed: nothing to do when no frame did).
-__global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32_t nGroupsStrict, int routed)
+// Frame-wide floods by one thread per frame, the steps FrameFlood follows (the CPU emulation runs this form): every
+// frame or only the frames that failed the exactness test of their per-component floods (routed).
+__global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32_t nFrames, int routed)
 {
 	PTB_AFTER_PREVIOUS();
 	__shared__ FloodSmem sm;
 	if (routed && ws.cnt->nroute == 0) { return; }
-	const uint32_t n = nGroupsStrict ? nGroupsStrict : ws.cnt->nmulti;
-	for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
+	for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < nFrames; m += gridDim.x * blockDim.x) {
 		if (routed && ws.frameRoute[m] == 0) { continue; }
 		const uint32_t nSeeds = ws.gSeedOff[m + 1] - ws.gSeedOff[m];
 		uint32_t* seeds = ws.gSeed + ws.gSeedOff[m];
 		SortSlice(seeds, nSeeds);
 		FloodGroupGlobal<false>(ws, seeds, nSeeds, ws.heapKey + ws.gOff[m], ws.heapPix + ws.gOff[m], sm);
+	}
+}
+
+// ---- Frame-wide flood by a warp -----------------------------------------------------------------------------------
+// A whole frame's flood (a routed frame, or every frame in strict mode) with its open entries in a 32-ary heap, its
+// first 16384 entries in shared memory: a level of a pop is one minimum over the lanes, three levels hold 32 768
+// entries, and eight lanes look at the popped pixel's neighbours while the heap is put in order. Equal keys (popped one
+// after the other; three frames in four have two equal seeds) end it, and the frame is flooded again with the binary
+// heap (FloodBinary). Bound: the serial chain of pops, about 1.5 us each (the neighbours come from L2). A 1024 x 1024
+// frame of 47 000 domain pixels takes 70 ms, with a tie 120-160 ms; one thread with the heap in global memory took 285 ms.
+constexpr size_t kFrameHeapBytes = kFrameHeap * (sizeof(unsigned long long) + sizeof(uint32_t));
+constexpr unsigned long long kNoKey = ~0ull;
+
+// Entries 0 .. kFrameHeap - 1 lie in shared memory, the rest in the group's slice of global memory.
+struct WideHeap {
+	unsigned long long* key;
+	uint32_t* pix;
+	unsigned long long* gkey;
+	uint32_t* gpix;
+	uint32_t len;
+
+	__device__ __forceinline__ unsigned long long& K(uint32_t i) const { return i < kFrameHeap ? key[i] : gkey[i]; }
+	__device__ __forceinline__ uint32_t& P(uint32_t i) const { return i < kFrameHeap ? pix[i] : gpix[i]; }
+
+	// Called by the whole warp with the same entry.
+	__device__ __forceinline__ void Push(unsigned long long k, uint32_t v)
+	{
+		const bool first = (threadIdx.x & 31) == 0;
+		uint32_t hole = len++;
+		while (hole > 0) {
+			const uint32_t parent = (hole - 1) / 32;
+			const unsigned long long pk = K(parent);
+			if (pk <= k) { break; }
+			const uint32_t pv = P(parent);
+			__syncwarp();
+			if (first) {
+				K(hole) = pk;
+				P(hole) = pv;
+			}
+			hole = parent;
+			__syncwarp();
+		}
+		if (first) {
+			K(hole) = k;
+			P(hole) = v;
+		}
+		__syncwarp();
+	}
+
+	// Removes the top (read before).
+	__device__ __forceinline__ void Drop()
+	{
+		const uint32_t lane = threadIdx.x & 31;
+		const unsigned long long last = K(--len);
+		const uint32_t lastPix = P(len);
+		uint32_t hole = 0;
+		__syncwarp();
+		while (32 * hole + 1 < len) {
+			const uint32_t child = 32 * hole + 1 + lane;
+			const unsigned long long k = child < len ? K(child) : kNoKey;
+			const uint32_t hi = WarpMin(static_cast<uint32_t>(k >> 32));
+			const uint32_t lo = WarpMin(static_cast<uint32_t>(k >> 32) == hi ? static_cast<uint32_t>(k) : 0xffffffffu);
+			const unsigned long long best = static_cast<unsigned long long>(hi) << 32 | lo;
+			if (best >= last) { break; }
+			const uint32_t holder = static_cast<uint32_t>(__ffs(__ballot_sync(0xffffffffu, k == best)) - 1);
+			if (lane == holder) {
+				K(hole) = k;
+				P(hole) = P(child);
+			}
+			hole = 32 * hole + 1 + holder;
+			__syncwarp();
+		}
+		if (lane == 0 && len > 0) {
+			K(hole) = last;
+			P(hole) = lastPix;
+		}
+		__syncwarp();
+	}
+};
+
+// What the frame-wide floods know of a frame: its pixels, its seeds and the neighbour each of eight lanes looks at.
+struct FrameView {
+	const Workspace& ws;
+	const uint32_t* pix;
+	uint32_t nPix, nSeeds;
+	int dr, dc;
+
+	__device__ __forceinline__ FrameView(const Workspace& w, int f) : ws(w)
+	{
+		const int lane = threadIdx.x & 31;
+		pix = ws.gPix + ws.gOff[f];
+		nPix = ws.gOff[f + 1] - ws.gOff[f];
+		nSeeds = ws.gSeedOff[f + 1] - ws.gSeedOff[f];
+		dr = lane < 3 ? -1 : (lane < 5 ? 0 : 1);
+		dc = lane < 3 ? lane - 1 : (lane < 5 ? (lane == 3 ? -1 : 1) : lane - 6);
+	}
+
+	// A labelled seed joins the flood when a neighbour in the frame is off the domain or unlabelled.
+	__device__ __forceinline__ bool Open(uint32_t s) const
+	{
+		const Pix q = Decompose(s, ws.g);
+		for (int t = 0; t < 9; ++t) {
+			const int yy = q.y + t / 3 - 1, xx = q.x + t % 3 - 1;
+			if (t == 4 || yy < 0 || yy >= ws.g.H || xx < 0 || xx >= ws.g.W) { continue; }
+			const uint32_t nb = s + static_cast<uint32_t>((t / 3 - 1) * ws.g.W + t % 3 - 1);
+			if (!(__ldg(ws.code + nb) & kDomain) || ws.lab[nb] == 0) { return true; }
+		}
+		return false;
+	}
+
+	__device__ __forceinline__ double SeedKey(uint32_t s) const { return -(static_cast<double>(__ldg(ws.w1 + s)) * kW1Unit); }
+
+	// This lane's neighbour nb of popped pixel p: whether p's pop pushes it, and its key. `order` puts the heap in order
+	// while the neighbour's data is on its way.
+	template <class Order>
+	__device__ __forceinline__ bool Look(uint32_t p, uint32_t pops, uint32_t& nb, double& key, Order order) const
+	{
+		const Pix q = Decompose(p, ws.g);
+		const int yy = q.y + dr, xx = q.x + dc;
+		nb = p + static_cast<uint32_t>(dr * ws.g.W + dc);
+		const bool in = (threadIdx.x & 31) < 8 && yy >= 0 && yy < ws.g.H && xx >= 0 && xx < ws.g.W;
+		const uint32_t code = in ? __ldg(ws.code + nb) : 0u, w = in ? __ldg(ws.w1 + nb) : 0u, lb = in ? ws.lab[nb] : 1u;
+		const uint32_t L = ws.lab[p];
+		order();
+		// key = -v + it * EPSILON, both operations rounded separately as in the reference
+		key = __dadd_rn(-(static_cast<double>(w) * kW1Unit), __dmul_rn(static_cast<double>(pops), kEps));
+		const bool push = (code & kDomain) != 0 && lb == 0;
+		if (push) { ws.lab[nb] = L; }
+		return push;
+	}
+
+	__device__ __forceinline__ void Unlabel() const
+	{
+		__syncwarp();
+		for (uint32_t i = threadIdx.x & 31; i < nPix; i += 32) {
+			if (!(__ldg(ws.code + pix[i]) & kSeed)) { ws.lab[pix[i]] = 0u; }
+		}
+		__syncwarp();
+	}
+};
+
+// The flood with the wide heap; false on a tie.
+__device__ bool FloodWide(const FrameView& v, const uint32_t* seeds, uint32_t* smem, double* hk, uint32_t* hp)
+{
+	const uint32_t lane = threadIdx.x & 31;
+	WideHeap heap{reinterpret_cast<unsigned long long*>(smem), smem + 2 * kFrameHeap, reinterpret_cast<unsigned long long*>(hk), hp, 0};
+	auto push = [&](bool pred, double key, uint32_t at) {
+		const unsigned long long k = KeyOrder(key);
+		for (unsigned m = __ballot_sync(0xffffffffu, pred); m != 0; m &= m - 1u) {
+			const int l = __ffs(m) - 1;
+			heap.Push(__shfl_sync(0xffffffffu, k, l), __shfl_sync(0xffffffffu, at, l));
+		}
+	};
+	for (uint32_t i0 = 0; i0 < v.nSeeds; i0 += 32) {
+		const uint32_t s = i0 + lane < v.nSeeds ? seeds[i0 + lane] : 0u;
+		const bool open = i0 + lane < v.nSeeds && v.Open(s);
+		push(open, open ? v.SeedKey(s) : 0.0, s);
+	}
+	unsigned long long before = kNoKey;
+	for (uint32_t pops = 1; heap.len > 0; ++pops) {
+		const unsigned long long top = heap.K(0);
+		const uint32_t p = heap.P(0);
+		if (top == before) { return false; }
+		before = top;
+		uint32_t nb;
+		double key;
+		const bool open = v.Look(p, pops, nb, key, [&]() { heap.Drop(); });
+		push(open, key, nb);
+	}
+	return true;
+}
+
+// The flood with libstdc++'s heap steps, which settle ties as the reference's queue does, by lane 0. Seeds are pushed in
+// raster order (sorted: room for them).
+__device__ void FloodBinary(const FrameView& v, const uint32_t* seeds, uint32_t* sorted, uint32_t* smem, double* hk, uint32_t* hp)
+{
+	const uint32_t lane = threadIdx.x & 31;
+	for (uint32_t i = lane; i < v.nSeeds; i += 32) {
+		const uint32_t s = seeds[i];
+		uint32_t rank = 0;
+		for (uint32_t k = 0; k < v.nSeeds; ++k) { rank += seeds[k] < s ? 1u : 0u; }
+		sorted[rank] = s;
+	}
+	__syncwarp();
+	SplitHeap heap{{{reinterpret_cast<double*>(smem), smem + 2 * kFrameHeap, 0, 1, 0xffffffffu, hk, hp}}};
+	uint32_t len = 0;
+	auto push = [&](bool pred, double key, uint32_t at) {
+		unsigned m = __ballot_sync(0xffffffffu, pred);
+		len += static_cast<uint32_t>(__popc(m));
+		for (; m != 0; m &= m - 1u) {
+			const int l = __ffs(m) - 1;
+			const double k = __shfl_sync(0xffffffffu, key, l);
+			const uint32_t a = __shfl_sync(0xffffffffu, at, l);
+			if (lane == 0) { heap.Push(k, a); }
+		}
+		__syncwarp();
+	};
+	for (uint32_t i0 = 0; i0 < v.nSeeds; i0 += 32) {
+		const uint32_t s = i0 + lane < v.nSeeds ? sorted[i0 + lane] : 0u;
+		const bool open = i0 + lane < v.nSeeds && v.Open(s);
+		push(open, open ? v.SeedKey(s) : 0.0, s);
+	}
+	for (uint32_t pops = 1; len > 0; ++pops) {
+		const uint32_t p = smem[2 * kFrameHeap];
+		__syncwarp();
+		--len;
+		uint32_t nb;
+		double key;
+		const bool open = v.Look(p, pops, nb, key, [&]() {
+			if (lane == 0) { heap.Pop(); }
+		});
+		push(open, key, nb);
+	}
+}
+
+// routed: only the frames flooded again frame-wide.
+__global__ void __launch_bounds__(32) FrameFlood(Workspace ws, int routed)
+{
+	PTB_AFTER_PREVIOUS();
+	extern __shared__ uint32_t frameHeap[];
+	if (routed && ws.cnt->nroute == 0) { return; }
+	for (int f = static_cast<int>(blockIdx.x); f < ws.g.B; f += static_cast<int>(gridDim.x)) {
+		if (routed && ws.frameRoute[f] == 0) { continue; }
+		const FrameView v(ws, f);
+		const uint32_t* seeds = ws.gSeed + ws.gSeedOff[f];
+		double* hk = ws.heapKey + ws.gOff[f];
+		uint32_t* hp = ws.heapPix + ws.gOff[f];
+		if (!FloodWide(v, seeds, frameHeap, hk, hp)) {
+			v.Unlabel();
+			// par is dead in a frame flooded as one unit: room for the seeds in order
+			FloodBinary(v, seeds, ws.par + static_cast<size_t>(f) * static_cast<size_t>(ws.g.N), frameHeap, hk, hp);
+		}
+		__syncwarp();
 	}
 }
 
@@ -979,7 +1233,7 @@ __device__ void FloodBox(BoxSmem& sm, const Geometry& geo, int bx0, int by0, int
 	__syncwarp();
 	if (lane == 0) {
 		SortSlice(seeds, nSeeds);
-		Heap heap{sm.key, sm.pix, 0, 1, kBoxHeap, hk, hp};
+		Heap heap{{sm.key, sm.pix, 0, 1, kBoxHeap, hk, hp}};
 		FloodGroup<true>(geo, BoxView{sm, bx0, by0, bw}, seeds, nSeeds, heap);
 	}
 	__syncwarp();
@@ -1031,7 +1285,7 @@ __global__ void __launch_bounds__(kBoxWarps * 32) GroupFloodBox(Workspace ws, in
 			__syncwarp();
 			if (lane == 0 && nPix > 0) {
 				SortSlice(seeds, nSeeds);
-				Heap heap{sm.key, sm.pix, 0, 1, kBoxHeap, hk, hp};
+				Heap heap{{sm.key, sm.pix, 0, 1, kBoxHeap, hk, hp}};
 				FloodGroup<true>(geo, GlobalView{ws}, seeds, nSeeds, heap);
 			}
 			__syncwarp();
@@ -1571,20 +1825,9 @@ __global__ void SuspectCount(Workspace ws)
 	}
 }
 
-// A frame that failed the rank test: flooded again per component with estimated frame-wide aging (reflood), or
-// routed to the frame-wide flood.
-__device__ __forceinline__ void FailRankTest(const Workspace& ws, int f, int reflood)
-{
-	if (!reflood) {
-		RouteFrame(ws, f, kRouteRankFused);
-		return;
-	}
-	if (atomicExch(ws.frameReflood + f, 1u) == 0u) { atomicAdd(&ws.cnt->nreflood, 1u); }
-}
-
-// Step 3: the rank test of every counted pair. reflood: frames that fail it are flooded again per component with
-// estimated frame-wide aging (no basin fusion follows); else they are routed to the frame-wide flood.
-__global__ void SuspectCheck(Workspace ws, int reflood)
+// Step 3: the rank test of every counted pair; a frame that fails it is flooded again per component with estimated
+// frame-wide aging.
+__global__ void SuspectCheck(Workspace ws, int)
 {
 	PTB_AFTER_PREVIOUS();
 	if (ws.cnt->nsuspect == 0) { return; }
@@ -1595,7 +1838,7 @@ __global__ void SuspectCheck(Workspace ws, int reflood)
 		const long long bc = ws.rankCount[2 * i];
 		const long long az = r.w == 0u ? 0ll : static_cast<long long>(ws.rankCount[2 * i + 1]) + 1;
 		const long long lhs = (static_cast<long long>(r.y) - static_cast<long long>(r.z)) * 78125ll;
-		if (!(lhs > (bc - az + 1) * 512ll)) { FailRankTest(ws, static_cast<int>(r.x), reflood); }
+		if (!(lhs > (bc - az + 1) * 512ll) && atomicExch(ws.frameReflood + r.x, 1u) == 0u) { atomicAdd(&ws.cnt->nreflood, 1u); }
 	}
 }
 
@@ -1622,7 +1865,7 @@ __global__ void __launch_bounds__(kPlanThreads) RefloodPlan(Workspace ws)
 	if (threadIdx.x == 0) {
 		for (int f = 0; f < ws.g.B; ++f) {
 			if (ws.frameReflood[f] == 0u) { continue; }
-			if (next < kRefloodSlots && ws.frameRoute[f] == 0u && ws.frameDom[f] <= kRefloodCap) {
+			if (next < RefloodSlots(ws.g) && ws.frameRoute[f] == 0u && ws.frameDom[f] <= kRefloodCap) {
 				ws.frameReflood[f] = next + 1u;
 				ws.rfInfo[next * 8 + 2] = static_cast<uint32_t>(f) + 1u;
 				++next;
@@ -1667,7 +1910,8 @@ __global__ void RefloodGather(Workspace ws)
 	// 16-pixel runs per frame, rounded up to whole warps: a warp never spans two slots, so it takes every branch below
 	// as one
 	const uint32_t per = ((N + 15u) / 16u + 31u) & ~31u;
-	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < kRefloodSlots * per; t += stride) {
+	const uint32_t slots = min(ws.cnt->nreflood, RefloodSlots(ws.g));  // taken in order from the first
+	for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < slots * per; t += stride) {
 		const uint32_t slot = t / per, q = t - slot * per;
 		const uint32_t f1 = ws.rfInfo[slot * 8 + 2];  // frame + 1 (0: the slot is unused)
 		if (f1 == 0u) { continue; }
@@ -1905,7 +2149,7 @@ __device__ bool RefloodGroupGlobal(const Workspace& ws, RfBoxSmem& sm, uint32_t 
 		uint32_t* seeds = ws.gSeed + ws.gSeedOff[m];
 		const uint32_t nSeeds = ws.gSeedOff[m + 1] - ws.gSeedOff[m];
 		SortSlice(seeds, nSeeds);
-		Heap heap{sm.key, sm.pix, 0, 1, kBoxHeap, ws.heapKey + off, ws.heapPix + off};
+		Heap heap{{sm.key, sm.pix, 0, 1, kBoxHeap, ws.heapKey + off, ws.heapPix + off}};
 		auto open = [&](uint32_t p, int y, int x) {
 			for (int dy = -1; dy <= 1; ++dy) {
 				const int yy = y + dy;
@@ -2073,7 +2317,7 @@ __global__ void __launch_bounds__(kRfWarps * 32) RefloodBox(Workspace ws)
 		}
 		if (!done && lane == 0) {
 			SortSlice(seeds, nSeeds);
-			Heap heap{sm.key, sm.pix, 0, 1, kBoxHeap, ws.heapKey + off, ws.heapPix + off};
+			Heap heap{{sm.key, sm.pix, 0, 1, kBoxHeap, ws.heapKey + off, ws.heapPix + off}};
 			auto at = [&](int y, int x) { return (y - by0) * bw + (x - bx0); };
 			for (uint32_t k = 0; k < nSeeds; ++k) {
 				const uint32_t sd = seeds[k];
@@ -2339,41 +2583,47 @@ bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPo
 		scan({{ws.gOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr}, {ws.gSeedOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr},
 		      {ws.gRegOff, &ws.cnt->nmulti, 0, ws.capComp, nullptr}}, groupState);
 	}
+	// frame-wide groups: a warp per frame
+	auto frameFlood = [&](int routed) {
+		static const bool heapSmem = PTB_CUDA(cudaFuncSetAttribute(FrameFlood, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                                           static_cast<int>(kFrameHeapBytes)));
+		ok = ok && heapSmem && LaunchChained(FrameFlood, static_cast<int>(std::min<uint32_t>(frames, 148u)), 32, kFrameHeapBytes, st, ws, routed);
+		CountLaunch();
+	};
 	launch(GroupScatter, grid, kThreads, strict ? 1 : 0);
-	if (strict) {  // frame-wide groups: one thread per group, small CTAs so that many SMs share the frames
-		launch(GroupFlood, grid * 2, kFloodThreads, groupsStrict, 0);
+	if (strict) {
+		frameFlood(0);
 	}
 	else {  // one warp per group, staged in shared memory
 		launch(GroupFloodBox, grid, kBoxWarps * 32, rank);
 	}
+	if (!strict && rank) {
+		// boundary pairs that failed the first exactness test: the rank test of their frames (each kernel returns at
+		// once when no pair failed), and the re-flood of those that fail it, with estimated frame-wide aging
+		launch(SuspectPlan, 1, kPlanThreads);
+		launch(SuspectCount, grid, kThreads);
+		launch(SuspectCheck, std::min(grid, 64), kThreads, 0);
+		launch(RefloodPlan, 1, kPlanThreads);
+		launch(RefloodGather, grid, kThreads);
+		static const bool bucketSmem = PTB_CUDA(cudaFuncSetAttribute(RefloodBucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                                             static_cast<int>(kRfBucketSmem)));
+		ok = ok && bucketSmem && LaunchChained(RefloodBucket, RefloodSlots(g) * 2, kRfBucketThreads, kRfBucketSmem, st, ws);
+		CountLaunch();
+		launch(RefloodCounts, grid, kThreads);
+		launch(RefloodBox, grid, kRfWarps * 32);
+	}
+	// the fusion takes the labels proven by then; frames routed so far are flooded and fused again frame-wide below
 	const bool fuse = static_cast<int>(ratio) > 0;  // WatershedIntelligent, Segmentation2D.cpp:77-85
 	if (fuse) {
 		if (!strict) { launch(GroupFuseBox, grid, kFuseWarps * 32, ratio); }
 		launch(GroupFuse, grid * 2, kFloodThreads, groupsStrict, ratio, 0);
 	}
 	if (!strict) {
-		// boundary pairs that failed the first exactness test: the rank test of their frames (each kernel returns at
-		// once when no pair failed)
-		if (rank) {
-			launch(SuspectPlan, 1, kPlanThreads);
-			launch(SuspectCount, grid, kThreads);
-			// frames failing the rank test: flooded again with estimated frame-wide aging (not after a basin fusion,
-			// which used the first flood's labels)
-			launch(SuspectCheck, std::min(grid, 64), kThreads, fuse ? 0 : 1);
-			launch(RefloodPlan, 1, kPlanThreads);
-			launch(RefloodGather, grid, kThreads);
-			static const bool bucketSmem = PTB_CUDA(cudaFuncSetAttribute(RefloodBucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                                             static_cast<int>(kRfBucketSmem)));
-			ok = ok && bucketSmem && LaunchChained(RefloodBucket, kRefloodSlots * 2, kRfBucketThreads, kRfBucketSmem, st, ws);
-			CountLaunch();
-			launch(RefloodCounts, grid, kThreads);
-			launch(RefloodBox, grid, kRfWarps * 32);
-		}
 		// frames whose per-component floods failed the exactness tests: flooded again as one unit with the frame-global
 		// pop counter (each kernel returns at once when no frame was routed)
 		launch(RedoOffsets, 1, kRedoThreads);
 		launch(GroupScatter, grid, kThreads, 2);
-		launch(GroupFlood, grid * 2, kFloodThreads, frames, 1);
+		frameFlood(1);
 		if (fuse) { launch(GroupFuse, grid * 2, kFloodThreads, frames, ratio, 1); }
 	}
 	launch(RegionStats, grid, kThreads);

@@ -7,6 +7,8 @@
 #include "engine.h"
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <condition_variable>
 #include <cstring>
@@ -24,6 +26,8 @@ bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPo
 bool LaunchBuildCandidates(const Workspace& ws, cudaStream_t st);
 bool LaunchSortFrames(const Workspace& ws, double* out, unsigned long long* rowBase, bool offsetOut, unsigned long long planeBase,
                       cudaStream_t st);
+bool LaunchCellTable(const double* given, double* cells64, float* cells32, size_t cells, cudaStream_t st);
+bool LaunchSwapTable(const double* given, double* swapped, int sx, int sy, long long slabs, cudaStream_t st);
 bool LaunchFit(const uint16_t* img, int H, int W, long long N, const Cand* cands, const uint32_t* nptr, uint32_t nconst,
                uint32_t cap, const FitParams& fp, double* rows, uint8_t* flags, int precision, cudaStream_t st);
 bool LaunchAstigEstimate(const double* dIn, double* dOut, uint64_t n, double pixelSize, const double* model, double zMax, cudaStream_t st);
@@ -52,9 +56,10 @@ bool CheckCuda(cudaError_t e, const char* what, const char* file, int line)
 }
 
 // ---- fit parameters ------------------------------------------------------------------------------------------
-bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, std::vector<double>& splineHost)
+bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, const double** splineTable)
 {
 	out = FitParams{};
+	*splineTable = nullptr;
 	out.mode = (fit >= 1 && fit <= 8) ? static_cast<int>(fit) : kNone;
 	out.sigmaX = 1.0;
 	out.sigmaY = 2.0;
@@ -89,7 +94,7 @@ bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, std::vector<
 			out.sx = m.sx; out.sy = m.sy; out.sz = m.sz;
 			out.splineSize = static_cast<long long>(m.sx) * m.sy * m.sz;
 			if (m.sx <= 0 || m.sy <= 0 || m.sz <= 0) { SetError("spline dimensions must be positive"); return false; }
-			splineHost.assign(fp + 9, fp + 9 + static_cast<size_t>(out.splineSize) * 64);
+			*splineTable = fp + 9;
 		}
 		if (roi % 2 == 0) { roi--; }
 		m.roi = roi;
@@ -117,9 +122,8 @@ bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, std::vector<
 			return false;
 		}
 		out.splineSize = static_cast<long long>(out.sx) * out.sy * out.sz;
-		const size_t ncoef = static_cast<size_t>(out.splineSize) * 64;
-		splineHost.assign(fp + 5, fp + 5 + ncoef);
-		const double centre = splineHost[(32 * static_cast<size_t>(out.splineSize)) + (out.sz / 2 * static_cast<size_t>(out.sx) * out.sy) +
+		*splineTable = fp + 5;
+		const double centre = fp[5 + (32 * static_cast<size_t>(out.splineSize)) + (out.sz / 2 * static_cast<size_t>(out.sx) * out.sy) +
 		                                 (out.sy / 2 * static_cast<size_t>(out.sx)) + (out.sx / 2)];
 		out.intensityRatio = std::abs(centre) < 2.220446049250313e-16 ? 1.0 : 4.0 / centre;
 		out.offsetXY = static_cast<long long>(std::floor((static_cast<double>(out.sx) + 1.0 - static_cast<double>(roi)) / 2));
@@ -193,23 +197,127 @@ cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
 	return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
-// Host memcpy over several threads (pageable buffers go through pinned staging; one thread copies about 10 GB/s).
+namespace {
+
+// Threads that help with host copies, shared by every engine of the process: started with the first large copy. One
+// thread moves 14-19 GB/s between pageable and pinned memory, eight of them 100 (a B200 host's 16 threads), the link 54.
+// A copy comes as a chain of short jobs, so a helper looks for the next one for a while before it sleeps, and the
+// caller waits for the last tasks without sleeping: waking either takes longer than a job.
+class CopyThreads {
+public:
+	static CopyThreads& Get()
+	{
+		static CopyThreads t;
+		return t;
+	}
+
+	// Calls task(0) .. task(n - 1) on the helpers and the calling thread; returns when all have finished.
+	void Run(size_t n, const std::function<void(size_t)>& task)
+	{
+		auto job = std::make_shared<Job>(n, &task);
+		bool sleeping = false;
+		{
+			std::lock_guard<std::mutex> lock(mu_);
+			jobs_.push_back(job);
+			posted_.fetch_add(1);
+			sleeping = asleep_ > 0;
+		}
+		if (sleeping) { wake_.notify_all(); }
+		Work(*job);
+		while (job->done.load() < n) { std::this_thread::yield(); }
+		std::lock_guard<std::mutex> lock(mu_);
+		jobs_.erase(std::find(jobs_.begin(), jobs_.end(), job));
+	}
+
+private:
+	struct Job {
+		Job(size_t count, const std::function<void(size_t)>* t) : n(count), task(t) {}
+		const size_t n;
+		const std::function<void(size_t)>* task;  // valid while the job has unfinished tasks
+		std::atomic<size_t> next{0}, done{0};
+	};
+	static constexpr std::chrono::microseconds kLook{200};
+
+	CopyThreads()
+	{
+		const unsigned hw = std::thread::hardware_concurrency();
+		try {
+			for (unsigned i = 0; i + 1 < std::min(8u, hw / 2); ++i) { threads_.emplace_back([this] { Loop(); }); }
+		}
+		catch (...) {
+			// fewer helpers, or none: the calling thread does the work
+		}
+	}
+
+	~CopyThreads()
+	{
+		{
+			std::lock_guard<std::mutex> lock(mu_);
+			stop_ = true;
+			posted_.fetch_add(1);
+		}
+		wake_.notify_all();
+		for (auto& t : threads_) { t.join(); }
+	}
+
+	static void Work(Job& job)
+	{
+		for (size_t i; (i = job.next.fetch_add(1)) < job.n;) {
+			(*job.task)(i);
+			job.done.fetch_add(1);
+		}
+	}
+
+	void Loop()
+	{
+		for (;;) {
+			std::shared_ptr<Job> job;
+			uint64_t seen = 0;
+			{
+				std::lock_guard<std::mutex> lock(mu_);
+				if (stop_) { return; }
+				seen = posted_.load();
+				for (auto& j : jobs_) {
+					if (j->next.load() < j->n) { job = j; }
+				}
+			}
+			if (job) {
+				Work(*job);
+				continue;
+			}
+			const auto until = std::chrono::steady_clock::now() + kLook;
+			while (posted_.load() == seen && std::chrono::steady_clock::now() < until) { std::this_thread::yield(); }
+			std::unique_lock<std::mutex> lock(mu_);
+			if (posted_.load() != seen) { continue; }
+			++asleep_;
+			wake_.wait(lock, [&] { return posted_.load() != seen; });
+			--asleep_;
+		}
+	}
+
+	std::mutex mu_;
+	std::condition_variable wake_;
+	std::vector<std::shared_ptr<Job>> jobs_;
+	std::vector<std::thread> threads_;
+	std::atomic<uint64_t> posted_{0};
+	int asleep_ = 0;
+	bool stop_ = false;
+};
+
+}  // namespace
+
+// Host memcpy, in pieces over several threads where it is long enough to be worth waking them.
 void ParallelCopy(void* dst, const void* src, size_t bytes)
 {
-	const size_t piece = 32ull << 20;
-	const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-	const unsigned n = static_cast<unsigned>(std::min<size_t>(hw, (bytes + piece - 1) / piece));
-	if (n <= 1) {
+	constexpr size_t kPiece = 128 << 10;
+	if (bytes < 4 * kPiece) {
 		std::memcpy(dst, src, bytes);
 		return;
 	}
-	std::vector<std::thread> th;
-	const size_t each = (bytes / n + 63) & ~static_cast<size_t>(63);
-	for (unsigned i = 0; i < n; ++i) {
-		const size_t a = std::min(bytes, each * i), b = std::min(bytes, each * (i + 1));
-		if (b > a) { th.emplace_back([=] { std::memcpy(static_cast<char*>(dst) + a, static_cast<const char*>(src) + a, b - a); }); }
-	}
-	for (auto& t : th) { t.join(); }
+	CopyThreads::Get().Run((bytes + kPiece - 1) / kPiece, [&](size_t i) {
+		const size_t at = i * kPiece;
+		std::memcpy(static_cast<char*>(dst) + at, static_cast<const char*>(src) + at, std::min(kPiece, bytes - at));
+	});
 }
 
 // True for host memory that is neither page-locked nor registered with CUDA.
@@ -221,6 +329,65 @@ bool Pageable(const void* p)
 		return true;
 	}
 	return a.type == cudaMemoryTypeUnregistered;
+}
+
+bool Engine::RingReady()
+{
+	for (int i = 0; i < kRing; ++i) {
+		if (!ring_[i] && !PTB_CUDA(cudaMallocHost(&ring_[i], kRingBytes))) { return false; }
+		if (!ringEv_[i] && !PTB_CUDA(cudaEventCreateWithFlags(&ringEv_[i], cudaEventDisableTiming))) { return false; }
+	}
+	return true;
+}
+
+bool Engine::CopyIn(void* device, const void* host, size_t bytes, cudaStream_t st)
+{
+	if (bytes == 0) { return true; }
+	if (!Pageable(host)) { return PTB_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, st)); }
+	if (!RingReady()) { return false; }
+	// a short copy in a few pieces too: the link starts with the first
+	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));
+	for (size_t at = 0; at < bytes; at += piece) {
+		const size_t n = std::min(piece, bytes - at);
+		const int slot = static_cast<int>(ringNext_++ % kRing);
+		if (!PTB_CUDA(cudaEventSynchronize(ringEv_[slot]))) { return false; }
+		ParallelCopy(ring_[slot], static_cast<const char*>(host) + at, n);
+		if (!PTB_CUDA(cudaMemcpyAsync(static_cast<char*>(device) + at, ring_[slot], n, cudaMemcpyHostToDevice, st)) ||
+		    !PTB_CUDA(cudaEventRecord(ringEv_[slot], st))) {
+			return false;
+		}
+	}
+	return true;
+}
+
+bool Engine::CopyOut(void* host, const void* device, size_t bytes, cudaStream_t st)
+{
+	if (bytes == 0) { return true; }
+	if (!Pageable(host)) {
+		return PTB_CUDA(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, st)) && PTB_CUDA(cudaStreamSynchronize(st));
+	}
+	if (!RingReady()) { return false; }
+	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));
+	const uint64_t pieces = (bytes + piece - 1) / piece, first = ringNext_;
+	ringNext_ += pieces;
+	for (uint64_t i = 0; i < pieces + kRing - 1; ++i) {
+		if (i < pieces) {
+			const int slot = static_cast<int>((first + i) % kRing);
+			if (!PTB_CUDA(cudaEventSynchronize(ringEv_[slot])) ||
+			    !PTB_CUDA(cudaMemcpyAsync(ring_[slot], static_cast<const char*>(device) + i * piece, std::min(piece, bytes - i * piece),
+			                              cudaMemcpyDeviceToHost, st)) ||
+			    !PTB_CUDA(cudaEventRecord(ringEv_[slot], st))) {
+				return false;
+			}
+		}
+		if (i + 1 >= kRing) {  // the piece kRing - 1 back is moved on while the later ones arrive
+			const uint64_t j = i + 1 - kRing;
+			const int slot = static_cast<int>((first + j) % kRing);
+			if (!PTB_CUDA(cudaEventSynchronize(ringEv_[slot]))) { return false; }
+			ParallelCopy(static_cast<char*>(host) + j * piece, ring_[slot], std::min(piece, bytes - j * piece));
+		}
+	}
+	return true;
 }
 
 // Bytes of workspace for B frames of H x W with `rowsCap` fit rows.
@@ -336,6 +503,10 @@ Engine::~Engine()
 	}
 	if (pool_) { cudaFree(pool_); }
 	if (img_) { cudaFree(img_); }
+	for (int i = 0; i < kRing; ++i) {
+		if (ringEv_[i]) { cudaEventDestroy(ringEv_[i]); }
+		if (ring_[i]) { cudaFreeHost(ring_[i]); }
+	}
 	if (hostStage_) { cudaFreeHost(hostStage_); }
 	for (void* h : hostOut_) {
 		if (h) { cudaFreeHost(h); }
@@ -740,23 +911,14 @@ long long Engine::Localize(const uint16_t* input, bool inputOnDevice, double* ou
 	}
 	if (!Init()) { return -1; }
 	FitParams fp;
-	std::vector<double>& spline = splineIn_;
-	if (!ParseFitParams(fit, fitParams, fp, spline)) { return -1; }
-	if (!UploadSpline(fp, spline)) { return -1; }
+	const double* table = nullptr;
+	if (!ParseFitParams(fit, fitParams, fp, &table)) { return -1; }
+	if (!UploadSpline(fp, table)) { return -1; }
 	const int H = static_cast<int>(height), W = static_cast<int>(width);
 	const uint32_t maxPoints = static_cast<uint32_t>(std::min<uint64_t>(perPlane, 0xffffffffu));
-	// pageable host buffers: the frames are copied into pinned staging by several host threads (a page source), and
-	// the rows reach the caller's buffer through pinned staging the same way; a copy from or to pageable memory would
-	// otherwise go through the driver's single staging buffer and block this thread
-	PageSource pageableIn;
-	if (!source && !inputOnDevice && !outputOnDevice && Pageable(input)) {
-		const size_t frameElems = static_cast<size_t>(H) * W;
-		pageableIn = [input, frameElems](uint64_t z0, uint64_t n, uint16_t* dst) {
-			ParallelCopy(dst, input + z0 * frameElems, static_cast<size_t>(n) * frameElems * sizeof(uint16_t));
-			return true;
-		};
-		source = &pageableIn;
-	}
+	// pageable host buffers: the frames go through the pinned ring (CopyIn), and the rows reach the caller's buffer
+	// through pinned staging, both moved by several host threads; a copy from or to pageable memory would otherwise go
+	// through the driver's single staging buffer and block this thread
 	const bool stageOut = !outputOnDevice && Pageable(output);
 	struct Pending {
 		double* dst = nullptr;
@@ -807,21 +969,18 @@ long long Engine::Localize(const uint16_t* input, bool inputOnDevice, double* ou
 	// input of chunk k into its staging slot; the slot's previous chunk (k - imgSlots) must have finished reading it
 	auto copyIn = [&](uint64_t k) {
 		const int slot = imgSlotOf(k);
-		const uint16_t* src = source ? nullptr : input + first[k] * N;
+		uint16_t* stage = nullptr;
 		if (source) {
 			// the pinned host slot's previous frames (chunk k - 2) must have reached the device before it is refilled
-			uint16_t* stage = static_cast<uint16_t*>(hostStage_) + ((k & 1) ? N * B : 0);
+			stage = static_cast<uint16_t*>(hostStage_) + ((k & 1) ? N * B : 0);
 			if (k >= 2 && !PTB_CUDA(cudaEventSynchronize(h2d_[imgSlotOf(k - 2)]))) { return false; }
 			if (!(*source)(first[k], count[k], stage)) {
 				SetError("page source failed");
 				return false;
 			}
-			src = stage;
 		}
 		if (k >= imgSlots && !PTB_CUDA(cudaStreamWaitEvent(copy_, imgFree_[slot], 0))) { return false; }
-		if (!PTB_CUDA(cudaMemcpyAsync(imgSlot(slot), src, N * framesOf(k) * sizeof(uint16_t), cudaMemcpyHostToDevice, copy_))) {
-			return false;
-		}
+		if (!CopyIn(imgSlot(slot), source ? stage : input + first[k] * N, N * framesOf(k) * sizeof(uint16_t), copy_)) { return false; }
 		return PTB_CUDA(cudaEventRecord(h2d_[slot], copy_));
 	};
 	unsigned long long rows = 0;
@@ -1030,7 +1189,7 @@ void Engine::MleEvaluations(uint64_t* out, int n)
 	}
 }
 
-bool Engine::UploadSpline(FitParams& fp, const std::vector<double>& spline)
+bool Engine::UploadSpline(FitParams& fp, const double* table)
 {
 	if (fp.mode >= kG2Fixed) {
 		// [0] FP64 re-factorisation count, [1..2] work-queue counters of the persistent fit kernels
@@ -1041,70 +1200,26 @@ bool Engine::UploadSpline(FitParams& fp, const std::vector<double>& spline)
 		fp.mle.chunk = EnvChunk() ? EnvChunk() : 1;
 	}
 	if (fp.mode != kMleSpline && fp.mode != kSplineEmccd) { return true; }
-	// the same table as the last upload (a stack fitted chunk by chunk, or call after call): reuse the device copy
-	const bool same = spline_ && splineCacheMode_ == fp.mode && splineCache_.size() == spline.size() &&
-	                  std::memcmp(splineCache_.data(), spline.data(), spline.size() * sizeof(double)) == 0;
-	if (!same) { splineCacheMode_ = -1; }  // the device copy is about to change: no longer the cached table
-	if (fp.mode == kMleSpline) {
-		// cell-major copies of the [64][cell] table: FP64 first, then FP32
-		const size_t cells = static_cast<size_t>(fp.splineSize);
-		if (same) {
-			fp.mle.table64 = static_cast<const double*>(spline_);
-			fp.mle.table = reinterpret_cast<const float*>(static_cast<const char*>(spline_) + cells * 64 * sizeof(double));
-			return true;
-		}
-		std::vector<double> aos64(cells * 64);
-		std::vector<float> aos32(cells * 64);
-		for (size_t i = 0; i < 64; ++i) {
-			for (size_t c = 0; c < cells; ++c) {
-				aos64[c * 64 + i] = spline[i * cells + c];
-				aos32[c * 64 + i] = static_cast<float>(spline[i * cells + c]);
-			}
-		}
-		const size_t bytes64 = aos64.size() * sizeof(double), bytes32 = aos32.size() * sizeof(float);
-		const size_t bytes = bytes64 + bytes32;
-		if (bytes > splineBytes_) {
-			if (spline_) { cudaFree(spline_); spline_ = nullptr; splineBytes_ = 0; }
-			if (!PTB_CUDA(cudaMalloc(&spline_, bytes))) { return false; }
-			splineBytes_ = bytes;
-		}
-		char* base = static_cast<char*>(spline_);
-		if (!PTB_CUDA(cudaMemcpyAsync(base, aos64.data(), bytes64, cudaMemcpyHostToDevice, stream_))) { return false; }
-		if (!PTB_CUDA(cudaMemcpyAsync(base + bytes64, aos32.data(), bytes32, cudaMemcpyHostToDevice, stream_))) { return false; }
-		if (!PTB_CUDA(cudaStreamSynchronize(stream_))) { return false; }
-		fp.mle.table64 = reinterpret_cast<const double*>(base);
-		fp.mle.table = reinterpret_cast<const float*>(base + bytes64);
-		splineCache_ = spline;
-		splineCacheMode_ = fp.mode;
-		return true;
-	}
-	// the reference's [64][z][y][x] table with x and y exchanged: the spline fit's lanes read consecutive y cells
-	const size_t cells = static_cast<size_t>(fp.splineSize);
-	if (same) {
-		fp.coeffs = static_cast<const double*>(spline_);
-		return true;
-	}
-	std::vector<double> table(cells * 64);
-	const size_t sx = static_cast<size_t>(fp.sx), sy = static_cast<size_t>(fp.sy), slabs = 64 * static_cast<size_t>(fp.sz);
-	for (size_t k = 0; k < slabs; ++k) {
-		const double* src = spline.data() + k * sx * sy;
-		double* dst = table.data() + k * sx * sy;
-		for (size_t y = 0; y < sy; ++y) {
-			for (size_t x = 0; x < sx; ++x) { dst[x * sy + y] = src[y * sx + x]; }
-		}
-	}
-	const size_t bytes = table.size() * sizeof(double);
+	// the table as given, then in the layout the fit reads, made on the device: mode 8 cell-major in FP64 and FP32, mode
+	// 5 with x and y exchanged
+	const size_t cells = static_cast<size_t>(fp.splineSize), raw = cells * 64 * sizeof(double);
+	const size_t bytes = fp.mode == kMleSpline ? 2 * raw + raw / 2 : 2 * raw;
 	if (bytes > splineBytes_) {
 		if (spline_) { cudaFree(spline_); spline_ = nullptr; splineBytes_ = 0; }
 		if (!PTB_CUDA(cudaMalloc(&spline_, bytes))) { return false; }
 		splineBytes_ = bytes;
 	}
-	if (!PTB_CUDA(cudaMemcpyAsync(spline_, table.data(), bytes, cudaMemcpyHostToDevice, stream_))) { return false; }
-	if (!PTB_CUDA(cudaStreamSynchronize(stream_))) { return false; }
-	fp.coeffs = static_cast<const double*>(spline_);
-	splineCache_ = spline;
-	splineCacheMode_ = fp.mode;
-	return true;
+	double* given = static_cast<double*>(spline_);
+	double* made = given + cells * 64;
+	if (!CopyIn(given, table, raw, stream_) || (!Pageable(table) && !PTB_CUDA(cudaStreamSynchronize(stream_)))) { return false; }
+	if (fp.mode == kMleSpline) {
+		float* made32 = reinterpret_cast<float*>(made + cells * 64);
+		fp.mle.table64 = made;
+		fp.mle.table = made32;
+		return LaunchCellTable(given, made, made32, cells, stream_);
+	}
+	fp.coeffs = made;
+	return LaunchSwapTable(given, made, fp.sx, fp.sy, 64ll * fp.sz, stream_);
 }
 
 long long Engine::FitPositions(const uint16_t* input, const double* positions, uint64_t nPoints, double* output,
@@ -1113,9 +1228,9 @@ long long Engine::FitPositions(const uint16_t* input, const double* positions, u
 	if (nPoints == 0) { return 0; }
 	if (!Init()) { return -1; }
 	FitParams fp;
-	std::vector<double>& spline = splineIn_;
-	if (!ParseFitParams(fit, fitParams, fp, spline)) { return -1; }
-	if (!UploadSpline(fp, spline)) { return -1; }
+	const double* table = nullptr;
+	if (!ParseFitParams(fit, fitParams, fp, &table)) { return -1; }
+	if (!UploadSpline(fp, table)) { return -1; }
 	const size_t N = static_cast<size_t>(height) * width;
 	std::vector<Cand> cands(nPoints);
 	std::vector<double> localIdx(nPoints);
@@ -1145,7 +1260,7 @@ long long Engine::FitPositions(const uint16_t* input, const double* positions, u
 	}
 	const size_t imgBytes = N * planes * sizeof(uint16_t);
 	if (!ReserveImage(imgBytes)) { return -1; }
-	if (!PTB_CUDA(cudaMemcpyAsync(img_, input, imgBytes, cudaMemcpyHostToDevice, stream_))) { return -1; }
+	if (!CopyIn(img_, input, imgBytes, stream_)) { return -1; }
 	Cand* dCand = nullptr;
 	double* dRows = nullptr;
 	uint8_t* dFlag = nullptr;
@@ -1158,8 +1273,7 @@ long long Engine::FitPositions(const uint16_t* input, const double* positions, u
 	ok = ok && LaunchFit(static_cast<const uint16_t*>(img_), static_cast<int>(height), static_cast<int>(width),
 	                     static_cast<long long>(N), dCand, nullptr, static_cast<uint32_t>(nPoints), static_cast<uint32_t>(nPoints),
 	                     fp, dRows, dFlag, precision_, stream_);
-	ok = ok && PTB_CUDA(cudaMemcpyAsync(output, dRows, sizeof(double) * kCols * nPoints, cudaMemcpyDeviceToHost, stream_));
-	ok = ok && PTB_CUDA(cudaStreamSynchronize(stream_));
+	ok = ok && CopyOut(output, dRows, sizeof(double) * kCols * nPoints, stream_);
 	if (dCand) { cudaFreeAsync(dCand, stream_); }
 	if (dRows) { cudaFreeAsync(dRows, stream_); }
 	if (dFlag) { cudaFreeAsync(dFlag, stream_); }
@@ -1191,10 +1305,10 @@ bool Engine::Planes(const uint16_t* input, double* output, uint64_t height, uint
 	bool ok = true;
 	for (uint64_t z0 = 0; z0 < planes && ok; z0 += B) {
 		const uint64_t b = std::min<uint64_t>(B, planes - z0);
-		ok = ok && PTB_CUDA(cudaMemcpyAsync(img_, input + z0 * N, N * b * sizeof(uint16_t), cudaMemcpyHostToDevice, stream_));
+		ok = ok && CopyIn(img_, input + z0 * N, N * b * sizeof(uint16_t), stream_);
 		ok = ok && LaunchPlane(static_cast<const uint16_t*>(img_), dOut, static_cast<int>(height), static_cast<int>(width),
 		                       static_cast<int>(b), level, stream_);
-		ok = ok && PTB_CUDA(cudaMemcpyAsync(output + z0 * N, dOut, N * b * sizeof(double), cudaMemcpyDeviceToHost, stream_));
+		ok = ok && CopyOut(output + z0 * N, dOut, N * b * sizeof(double), stream_);
 	}
 	ok = ok && PTB_CUDA(cudaStreamSynchronize(stream_));
 	cudaFreeAsync(dOut, stream_);
@@ -1263,9 +1377,9 @@ bool Engine::Track(const double* input, uint64_t* output, uint64_t n, double max
 	uint64_t* dOut = nullptr;
 	bool ok = PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dIn), n * 4 * sizeof(double), stream_));
 	ok = ok && PTB_CUDA(ScratchAlloc(reinterpret_cast<void**>(&dOut), n * 2 * sizeof(uint64_t), stream_));
-	ok = ok && PTB_CUDA(cudaMemcpyAsync(dIn, input, n * 4 * sizeof(double), cudaMemcpyHostToDevice, stream_));
+	ok = ok && CopyIn(dIn, input, n * 4 * sizeof(double), stream_);
 	ok = ok && TrackDevice(dIn, dOut, n, maxDistance, stream_);
-	ok = ok && PTB_CUDA(cudaMemcpyAsync(output, dOut, n * 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, stream_));
+	ok = ok && CopyOut(output, dOut, n * 2 * sizeof(uint64_t), stream_);
 	if (dIn) { cudaFreeAsync(dIn, stream_); }
 	if (dOut) { cudaFreeAsync(dOut, stream_); }
 	return PTB_CUDA(cudaStreamSynchronize(stream_)) && ok;

@@ -17,7 +17,8 @@
 
 namespace ptb {
 
-bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, std::vector<double>& splineHost);
+// *splineTable: the coefficient table inside fp for the spline modes, else null.
+bool ParseFitParams(uint64_t fit, const double* fp, FitParams& out, const double** splineTable);
 long long FittingDeviceNoAlloc(const uint16_t* dStack, const double* dPositions, uint64_t nPoints, double* dOutput,
                                uint64_t height, uint64_t width, uint64_t planes, uint64_t fit, const double* fitParams,
                                int precision, int lanes, cudaStream_t st);
@@ -105,7 +106,13 @@ public:
 private:
 	bool Reserve(int H, int W, int B, uint32_t rowsCap, int slots);
 	bool ReserveImage(size_t bytes);
-	bool UploadSpline(FitParams& fp, const std::vector<double>& spline);
+	bool UploadSpline(FitParams& fp, const double* table);
+	// Copies between device memory and any host memory, ordered on st. Pageable memory goes through the pinned ring piece
+	// by piece, each moved by several host threads while the previous one is on the link; CopyOut returns when the data
+	// has arrived, CopyIn when the host memory has been read.
+	bool CopyIn(void* device, const void* host, size_t bytes, cudaStream_t st);
+	bool CopyOut(void* host, const void* device, size_t bytes, cudaStream_t st);
+	bool RingReady();
 	void TunedMapping(FitParams& fp, int sizeClass) const;
 	bool Autotune(FitParams& fp, const uint16_t* dImg, int H, int W, int slot, int sizeClass);
 	int ChunkFrames(int H, int W, uint64_t planes, uint32_t maxPoints, size_t budget) const;
@@ -160,15 +167,17 @@ private:
 	size_t poolBytes_ = 0;
 	void* img_ = nullptr;
 	size_t imgBytes_ = 0;
+	static constexpr int kRing = 4;
+	static constexpr size_t kRingBytes = 4ull << 20;
+	void* ring_[kRing] = {};                  // pinned staging of pageable host memory (CopyIn, CopyOut)
+	cudaEvent_t ringEv_[kRing] = {};          // the piece in the slot has crossed the link
+	uint64_t ringNext_ = 0;
 	void* hostStage_ = nullptr;               // pinned frame staging of page sources (two slots)
 	size_t hostStageBytes_ = 0;
 	void* hostOut_[2] = {};                   // pinned row staging for pageable output (two buffers)
 	size_t hostOutBytes_[2] = {};
 	cudaEvent_t outEv_[2] = {};               // a staged row copy reached hostOut_
-	void* spline_ = nullptr;
-	std::vector<double> splineIn_;            // the call's spline table as given (reused between calls)
-	std::vector<double> splineCache_;         // the table behind spline_ (its upload is skipped when unchanged)
-	int splineCacheMode_ = -1;
+	void* spline_ = nullptr;                  // the call's spline table as given and in the layouts the fits read
 	void* fallbacks_ = nullptr;
 	struct Tuned {
 		int key;    // (mode * 64 + roi) * 64 + chunk size class

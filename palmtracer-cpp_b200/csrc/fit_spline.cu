@@ -389,7 +389,55 @@ __global__ void __launch_bounds__(32 * kWarps, 3) SplineFitKernel(const uint16_t
 	}
 }
 
+// The table as given, [64][cells], in the layout the maximum-likelihood spline fit reads, [cells][64] in
+// FP64 and FP32: a tile of 32 cells per CTA, read along the cells and written along the coefficients.
+constexpr int kTableCells = 32;
+__global__ void __launch_bounds__(256) CellTable(const double* __restrict__ given, double* __restrict__ cells64,
+                                                 float* __restrict__ cells32, size_t cells)
+{
+	__shared__ double tile[64][kTableCells + 1];
+	const size_t c0 = static_cast<size_t>(blockIdx.x) * kTableCells;
+	for (int i = threadIdx.x; i < 64 * kTableCells; i += 256) {
+		const int k = i / kTableCells, c = i % kTableCells;
+		if (c0 + c < cells) { tile[k][c] = __ldg(given + k * cells + c0 + c); }
+	}
+	__syncthreads();
+	for (int i = threadIdx.x; i < 64 * kTableCells; i += 256) {
+		const int c = i / 64, k = i % 64;
+		if (c0 + c < cells) {
+			cells64[(c0 + c) * 64 + k] = tile[k][c];
+			cells32[(c0 + c) * 64 + k] = static_cast<float>(tile[k][c]);
+		}
+	}
+}
+
+__global__ void SwapTable(const double* __restrict__ given, double* __restrict__ swapped, int sx, int sy, long long n)
+{
+	const long long slab = static_cast<long long>(sx) * sy;
+	for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < n; k += gridDim.x * static_cast<long long>(blockDim.x)) {
+		const long long s = k / slab, r = k - s * slab;
+		const int x = static_cast<int>(r / sy), y = static_cast<int>(r - static_cast<long long>(x) * sy);
+		swapped[k] = __ldg(given + s * slab + static_cast<long long>(y) * sx + x);
+	}
+}
+
 }  // namespace
+
+bool LaunchCellTable(const double* given, double* cells64, float* cells32, size_t cells, cudaStream_t st)
+{
+	CellTable<<<static_cast<unsigned>((cells + kTableCells - 1) / kTableCells), 256, 0, st>>>(given, cells64, cells32, cells);
+	CountLaunch();
+	return PTB_LAUNCHED();
+}
+
+// The reference's table [slabs = 64 sz][sy][sx] as [slabs][sx][sy].
+bool LaunchSwapTable(const double* given, double* swapped, int sx, int sy, long long slabs, cudaStream_t st)
+{
+	const long long n = slabs * sx * sy;
+	SwapTable<<<static_cast<unsigned>(std::min<long long>((n + 255) / 256, 148 * 8)), 256, 0, st>>>(given, swapped, sx, sy, n);
+	CountLaunch();
+	return PTB_LAUNCHED();
+}
 
 bool LaunchSpline(const uint16_t* img, int H, int W, long long N, const Cand* cands, const uint32_t* nptr, uint32_t nconst,
                   uint32_t cap, const FitParams& fp, double* rows, cudaStream_t st)

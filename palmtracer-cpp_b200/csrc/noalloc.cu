@@ -149,8 +149,8 @@ long long FittingDeviceNoAlloc(const uint16_t* dStack, const double* dPositions,
 		return -1;
 	}
 	FitParams fp;
-	std::vector<double> unused;
-	if (!ParseFitParams(fit, fitParams, fp, unused)) { return -1; }
+	const double* table = nullptr;
+	if (!ParseFitParams(fit, fitParams, fp, &table)) { return -1; }
 	NoAllocScratch* s = ScratchForCurrentDevice();
 	if (s == nullptr) { return -1; }
 	fp.mle.fallbacks = &s->fallbacks;

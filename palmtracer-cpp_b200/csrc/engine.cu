@@ -26,7 +26,7 @@ bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPo
 bool LaunchBuildCandidates(const Workspace& ws, cudaStream_t st);
 bool LaunchSortFrames(const Workspace& ws, double* out, unsigned long long* rowBase, bool offsetOut, unsigned long long planeBase,
                       cudaStream_t st);
-bool LaunchCellTable(const double* given, double* cells64, float* cells32, size_t cells, cudaStream_t st);
+bool LaunchCellTable(const double* given, double* quads64, float* cells32, float* quads32, size_t cells, cudaStream_t st);
 bool LaunchSwapTable(const double* given, double* swapped, int sx, int sy, long long slabs, cudaStream_t st);
 bool LaunchFit(const uint16_t* img, int H, int W, long long N, const Cand* cands, const uint32_t* nptr, uint32_t nconst,
                uint32_t cap, const FitParams& fp, double* rows, uint8_t* flags, int precision, cudaStream_t st);
@@ -672,7 +672,7 @@ static std::vector<uint64_t> ChainKey(int slot, const Workspace& ws, const uint1
 	d(m.pixelSize); d(m.zMin); d(m.zMax);
 	for (double a : m.astig) { d(a); }
 	u(static_cast<uint64_t>(m.sx)); u(static_cast<uint64_t>(m.sy)); u(static_cast<uint64_t>(m.sz)); d(m.dz);
-	p(m.table); p(m.table64); p(m.fallbacks); p(m.queue); p(m.evals);
+	p(m.table); p(m.table64); p(m.tableQ); p(m.fallbacks); p(m.queue); p(m.evals);
 	return k;
 }
 
@@ -1200,10 +1200,10 @@ bool Engine::UploadSpline(FitParams& fp, const double* table)
 		fp.mle.chunk = EnvChunk() ? EnvChunk() : 1;
 	}
 	if (fp.mode != kMleSpline && fp.mode != kSplineEmccd) { return true; }
-	// the table as given, then in the layout the fit reads, made on the device: mode 8 cell-major in FP64 and FP32, mode
-	// 5 with x and y exchanged
+	// the table as given, then in the layout the fit reads, made on the device: mode 8 cell-major in FP32 and
+	// by x-monomials in FP32 and FP64, mode 5 with x and y exchanged
 	const size_t cells = static_cast<size_t>(fp.splineSize), raw = cells * 64 * sizeof(double);
-	const size_t bytes = fp.mode == kMleSpline ? 2 * raw + raw / 2 : 2 * raw;
+	const size_t bytes = fp.mode == kMleSpline ? 3 * raw : 2 * raw;
 	if (bytes > splineBytes_) {
 		if (spline_) { cudaFree(spline_); spline_ = nullptr; splineBytes_ = 0; }
 		if (!PTB_CUDA(cudaMalloc(&spline_, bytes))) { return false; }
@@ -1216,7 +1216,9 @@ bool Engine::UploadSpline(FitParams& fp, const double* table)
 		float* made32 = reinterpret_cast<float*>(made + cells * 64);
 		fp.mle.table64 = made;
 		fp.mle.table = made32;
-		return LaunchCellTable(given, made, made32, cells, stream_);
+		fp.mle.tableQ = made32 + cells * 64;
+		fp.mle.cells = fp.splineSize;
+		return LaunchCellTable(given, made, made32, made32 + cells * 64, cells, stream_);
 	}
 	fp.coeffs = made;
 	return LaunchSwapTable(given, made, fp.sx, fp.sy, 64ll * fp.sz, stream_);

@@ -18,7 +18,7 @@
 // Two mappings, chosen per (mode, ROI) by the autotuner in engine.cu:
 //   * thread per ROI, four launches that hand their state over in the output rows (columns 0-4 theta, column 5 a
 //     status) so that no extra device memory is needed:
-//       MleInitKernel   initial values and axial pre-scan;
+//       MleInitKernel   initial values (mode 6), MleScanKernel with the axial pre-scan (modes 7, 8);
 //       MleLmKernel     persistent FP32 LM: every warp owns a contiguous range of candidates and each lane takes the
 //                       next candidate of the range as soon as its own converges, so a lane never idles while the
 //                       other 31 iterate; ROI photons and the column erf factors are staged per lane in shared memory;
@@ -27,8 +27,8 @@
 //   * warp per ROI (MleWarpKernel): all four phases in one launch, pixels spread over the lanes, sums reduced with
 //     shuffles; better for large ROIs and for the spline model, whose 64 coefficients per pixel dominate.
 // For modes 6-7 the pixel-integrated Gaussian is separable: the erf factors are formed once per ROI column and row
-// per evaluation. The spline table is cell-major ([cell][64]) in FP32 for the FP32 phases and in FP64 for the FP64
-// ones.
+// per evaluation. The spline table is cell-major ([cell][64]) in FP32 for a thread per ROI, and for lane groups and the
+// FP64 pass by x-monomials, [16][cell][4] (SplinePixel).
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -221,7 +221,13 @@ __device__ __forceinline__ int SplineCell(float v, int dim) { return min(max(sta
 // Cubic-spline PSF at table coordinates (X, Y, Z): the cell index is clamped to the table and the fraction taken
 // from the clamped cell, as in the oracle. P1 and P2 are the derivatives in the fit parameters (x, y, s): X and Y
 // decrease as x and y grow, so their odd derivatives change sign.
-template <typename T, int NF>
+// L: lanes per ROI. A lane that walks its ROI's pixels alone reads a cell's coefficients in one run ([cell][64]). The
+// lanes of a group hold neighbouring pixels, whose cells are neighbours in x: in FP32 they read the four x-monomials of
+// one (z, y) pair from [16][cell][4], 16 bytes each and next to one another, 4 cache lines per 16 lanes. From the runs
+// every lane read a line of its own, and those lookups bound the fit (L1 97 % busy).
+// Measured, 94 152 ROIs of 13 x 13, whole localization: 16 lanes 20.5 ms from the runs, 14.1 ms from the monomials, 2 lanes
+// 19.1 and 15.3 ms (before the bounds on registers).
+template <typename T, int NF, int L>
 __device__ __forceinline__ T SplinePixel(const MleParams& mp, T X, T Y, T Z, T P1[3], T P2[6])
 {
 	const int ix = SplineCell(X, mp.sx), iy = SplineCell(Y, mp.sy), iz = SplineCell(Z, mp.sz);
@@ -239,12 +245,13 @@ __device__ __forceinline__ T SplinePixel(const MleParams& mp, T X, T Y, T Z, T P
 	for (int q = 0; q < 16; ++q) {  // q = zi * 4 + yj: the four x-monomials of one (z, y) pair
 		T c0, c1, c2, c3;
 		if constexpr (std::is_same<T, float>::value) {
-			const float4 c = __ldg(reinterpret_cast<const float4*>(mp.table + cell * 64) + q);
+			const float4 c = L >= 2 ? __ldg(reinterpret_cast<const float4*>(mp.tableQ) + q * mp.cells + cell)
+			                        : __ldg(reinterpret_cast<const float4*>(mp.table + cell * 64) + q);
 			c0 = c.x; c1 = c.y; c2 = c.z; c3 = c.w;
 		}
 		else {
-			const double2 a = __ldg(reinterpret_cast<const double2*>(mp.table64 + cell * 64) + 2 * q);
-			const double2 b = __ldg(reinterpret_cast<const double2*>(mp.table64 + cell * 64) + 2 * q + 1);
+			const double2* at = reinterpret_cast<const double2*>(mp.table64) + (q * mp.cells + cell) * 2;
+			const double2 a = __ldg(at), b = __ldg(at + 1);
 			c0 = a.x; c1 = a.y; c2 = b.x; c3 = b.y;
 		}
 		const int zi = q >> 2, yj = q & 3;
@@ -377,7 +384,7 @@ __device__ T Normal(const MleParams& mp, const Pix& px, const T th[5], T G[5], T
 		const int di = L / roi, dj = L - di * roi;
 		for (int k = gl; k < n; k += L) {
 			const T d = Photons<T>(px, i, j, k);
-			const T psf = SplinePixel<T, NF>(mp, X0 + T(j - h) - th[2], Y0 + T(i - h) - th[3], th[4], P1, P2);
+			const T psf = SplinePixel<T, NF, L>(mp, X0 + T(j - h) - th[2], Y0 + T(i - h) - th[3], th[4], P1, P2);
 			Accumulate<T, KIND>(d, th[0], th[1], psf, P1, P2, D, G, Hm, Fm);
 			i += di;
 			j += dj;
@@ -896,16 +903,12 @@ __device__ __forceinline__ uint32_t CandCount(const uint32_t* nptr, uint32_t nco
 // ---------------------------------------------------------------------------------------------------------------
 // Thread per ROI.
 
-// Initial values; shared memory: per thread the FP32 column factors of the axial pre-scan (roi floats).
-template <int MODEL>
+// Initial values of mode 6.
 __global__ void __launch_bounds__(kThreads) MleInitKernel(FitImages fi,
                                                           const Cand* __restrict__ cands, const uint32_t* nptr, uint32_t nconst,
                                                           MleParams mp, double* rows)
 {
-	extern __shared__ __align__(16) unsigned char smem[];
-	const FacTab<float> xt{reinterpret_cast<float*>(smem) + threadIdx.x, static_cast<int>(blockDim.x)};
 	const uint32_t n = CandCount(nptr, nconst);
-	unsigned long long evals = 0;
 	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		double* row = rows + static_cast<long long>(k) * kCols;
 		RoiAt r;
@@ -915,9 +918,97 @@ __global__ void __launch_bounds__(kThreads) MleInitKernel(FitImages fi,
 		}
 		const Pix px = MakePix(mp, r.base, r.W, nullptr, 0);
 		double t[5];
-		evals += InitTheta<MODEL, 1>(mp, px, r, t, xt, xt);
+		InitTheta<6, 1>(mp, px, r, t, FacTab<float>{nullptr, 0}, FacTab<float>{nullptr, 0});
 		#pragma unroll
 		for (int a = 0; a < 5; ++a) { row[a] = t[a]; }
+		row[kStatusCol] = kStOk;
+	}
+}
+
+// Initial values of modes 7 and 8: InitTheta with the axial pre-scan's points over the warps of a block that holds 32
+// ROIs, one per lane; each point's deviance is summed by one thread in pixel order, and the first smallest is taken. One
+// thread that made all of a ROI's evaluations left the SMs waiting (an instruction in 7 % of the cycles). The lanes of a
+// warp stay at one z and one pixel, so their spline cells coincide and the coefficient loads are broadcasts. Mode 7,
+// 215 770 ROIs of 11 x 11: 0.87 -> 0.52 ms; mode 8, 94 152 ROIs of 13 x 13: 1.93 -> 1.14 ms, where what is left is the
+// load of 256 bytes per pixel and lane.
+constexpr int kScanWarps = 8;
+template <int MODEL> struct ScanPoints { static constexpr int value = MODEL == 7 ? 16 : 8; };
+__host__ __device__ __forceinline__ int ScanSharedWords(int n, int roi, int model)
+{
+	return 32 * n + (model == 7 ? roi * 32 * kScanWarps : 0) + (n * 32 + 1) / 2;
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(32 * kScanWarps, MODEL == 8 ? 2 : 0) MleScanKernel(FitImages fi,
+                                                                 const Cand* __restrict__ cands, const uint32_t* nptr, uint32_t nconst,
+                                                                 MleParams mp, double* rows)
+{
+	constexpr int ns = ScanPoints<MODEL>::value;
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ float start[2][32], dev[ns][32];
+	float* ph = reinterpret_cast<float*>(smem);
+	float* fac = ph + 32 * mp.n;
+	uint16_t* raw = reinterpret_cast<uint16_t*>(fac + (MODEL == 7 ? mp.roi * 32 * kScanWarps : 0));
+	const int lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+	const FacTab<float> xt{fac + threadIdx.x, 32 * kScanWarps};
+	const uint32_t n = CandCount(nptr, nconst);
+	unsigned long long evals = 0;
+	for (uint32_t base = blockIdx.x * 32; base < n; base += gridDim.x * 32) {
+		const uint32_t k = base + lane;
+		RoiAt r;
+		const bool ok = k < n && Locate(fi, mp, cands[k], r);
+		Pix px = MakePix(mp, nullptr, 0, ph + lane, 32);
+		if (ok) {
+			for (int q = warp; q < mp.n; q += kScanWarps) {
+				const int i = q / mp.roi, j = q - i * mp.roi;
+				const uint16_t v = __ldg(r.base + i * r.W + j);
+				raw[q * 32 + lane] = v;
+				ph[q * 32 + lane] = fmaxf((float(v) - px.off32) * px.inv32, 0.f);
+			}
+		}
+		__syncthreads();
+		double t[5], lo[5], hi[5];
+		if (ok) {
+			Bounds<MODEL>(mp, r.x0, r.y0, lo, hi);
+			if (warp == 0) {
+				double dmin = 1e300, sum = 0;
+				for (int q = 0; q < mp.n; ++q) {
+					const double d = fmax((double(raw[q * 32 + lane]) - px.off64) * px.inv64, 0.0);
+					dmin = fmin(dmin, d);
+					sum += d;
+				}
+				t[0] = fmax(dmin, 1e-3);
+				t[1] = fmax(sum - t[0] * mp.n, 1.0);
+				start[0][lane] = float(t[0]);
+				start[1][lane] = float(t[1]);
+			}
+		}
+		__syncthreads();
+		if (ok) {
+			float tf[5] = {start[0][lane], start[1][lane], float(r.x0), float(r.y0), 0.f};
+			for (int s = warp; s < ns; s += kScanWarps) {
+				tf[4] = float(lo[4] + (hi[4] - lo[4]) * (s + 0.5) / ns);
+				dev[s][lane] = Normal<float, MODEL, 1, kDevOnly>(mp, px, tf, nullptr, nullptr, nullptr, xt, xt);
+			}
+		}
+		__syncthreads();
+		if (warp != 0 || k >= n) { continue; }
+		double* row = rows + static_cast<long long>(k) * kCols;
+		if (!ok) {
+			row[kStatusCol] = kStBorder;
+			continue;
+		}
+		t[2] = r.x0;
+		t[3] = r.y0;
+		float best = __int_as_float(0x7f800000);
+		t[4] = 0.5 * (lo[4] + hi[4]);
+		for (int s = 0; s < ns; ++s) {
+			const float D = dev[s][lane];
+			if (D < best) { best = D; t[4] = lo[4] + (hi[4] - lo[4]) * (s + 0.5) / ns; }
+		}
+		evals += ns;
+		#pragma unroll
+		for (int a = 0; a < 5; ++a) { row[a] = fmin(fmax(t[a], lo[a]), hi[a]); }
 		row[kStatusCol] = kStOk;
 	}
 	if (mp.evals && evals) { atomicAdd(mp.evals + 2, evals); }
@@ -1054,9 +1145,12 @@ struct SlotView {
 // Persistent FP32 LM (WarpQueue). Every pass of the loop makes each busy ROI evaluate the deviance, gradient and
 // Fisher matrix once: at the start point of a new candidate, or at the trial point of an LM step. L lanes per ROI
 // (1: a thread per ROI); the lanes of a group hold the same state and take the same branches. Shared memory per ROI
-// slot: the photons and the factor tables (SlotFloats, NF = 3).
+// slot: the photons and the factor tables (SlotFloats, NF = 3). The spline model's wide groups wait for their
+// coefficients (L1 hits 14 %): held to 128 registers, 8 blocks per SM instead of 6 at 130, 94 152 ROIs of 13 x 13 take
+// 3.95 ms instead of 6.70 with 16 lanes (10 and 12 blocks the same, 16 blocks spill: 4.43). Whole localization, without
+// and with the bound: 8 lanes 12.0 and 9.2 ms, 4 lanes 10.1 and 10.3, 2 lanes 14.9 and 19.4 (registers spilled).
 template <int MODEL, int L>
-__global__ void __launch_bounds__(kThreads) MleLmKernel(FitImages fi,
+__global__ void __launch_bounds__(kThreads, MODEL == 8 && L >= 8 ? 8 : 0) MleLmKernel(FitImages fi,
                                                         const Cand* __restrict__ cands, const uint32_t* nptr, uint32_t nconst,
                                                         MleParams mp, double* rows)
 {
@@ -1249,19 +1343,25 @@ __global__ void __launch_bounds__(kThreads, MODEL == 6 && L == 1 ? 8 : 0) MlePol
 	if (mp.evals && evals) { atomicAdd(mp.evals + 1, evals); }
 }
 
-// FP64 deviance, Fisher information and CRLB at the polished theta; writes the output row. Shared memory per thread:
-// the FP64 column factors (3 roi doubles). Mode 6 is held to 128 registers (8 blocks of 64 threads per SM), which it
-// fits without spilling; modes 7 and 8 keep the compiler's own allocation (a bound spills them).
-template <int MODEL>
-__global__ void __launch_bounds__(kThreads, MODEL == 6 ? 8 : 0) MleFinalKernel(FitImages fi,
+// FP64 deviance, Fisher information and CRLB at the polished theta; writes the output row. L lanes per ROI. Shared memory
+// for L = 1: per thread the FP64 column factors (3 roi doubles), lane-interleaved; L > 1: per group the column and row
+// factors (modes 6, 7). Modes 6 and 8 are held to 128 registers (8 blocks of 64 threads per SM), which they fit without
+// spilling; mode 7 keeps the compiler's own allocation (a bound spills it). Mode 8, 94 152 ROIs of 13 x 13: 2.12 ms with
+// one thread per ROI, 0.81 with 8 lanes (4: 0.84, 16: 0.85), 0.69 with the bound. Modes 6 and 7 are bound by their FP64
+// work and 4 lanes, which repeat the 5 x 5 inverse, are no faster (mode 6 0.79 -> 1.07 ms, mode 7 0.38 -> 0.36 ms).
+template <int MODEL, int L>
+__global__ void __launch_bounds__(kThreads, MODEL == 7 ? 0 : 8) MleFinalKernel(FitImages fi,
                                                            const Cand* __restrict__ cands, const uint32_t* nptr, uint32_t nconst,
                                                            MleParams mp, double* rows)
 {
 	extern __shared__ __align__(16) unsigned char smem[];
-	const FacTab<double> xt{reinterpret_cast<double*>(smem) + threadIdx.x, static_cast<int>(blockDim.x)};
+	double* tab = reinterpret_cast<double*>(smem) + (L == 1 ? threadIdx.x : threadIdx.x / L * 6 * mp.roi);
+	const FacTab<double> xt{tab, L == 1 ? static_cast<int>(blockDim.x) : 1};
+	const FacTab<double> yt{L == 1 ? tab : tab + 3 * mp.roi, xt.s};
+	const Group<L> grp;
 	const uint32_t n = CandCount(nptr, nconst);
 	unsigned long long evals = 0;
-	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+	for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) / L; k < n; k += gridDim.x * blockDim.x / L) {
 		double* row = rows + static_cast<long long>(k) * kCols;
 		const Cand cd = cands[k];
 		RoiAt r;
@@ -1270,12 +1370,13 @@ __global__ void __launch_bounds__(kThreads, MODEL == 6 ? 8 : 0) MleFinalKernel(F
 		if (ok) {
 			#pragma unroll
 			for (int a = 0; a < 5; ++a) { t[a] = row[a]; }
-			ok = Final<MODEL, 1>(mp, MakePix(mp, r.base, r.W, nullptr, 0), t, crlb, dev, xt, xt);
+			ok = Final<MODEL, L>(mp, MakePix(mp, r.base, r.W, nullptr, 0), t, crlb, dev, xt, yt);
 			++evals;
 		}
-		StoreMleRow(row, -1, mp, cd, t, crlb, dev, r.ux, r.uy, ok);
+		if constexpr (L > 1) { __syncwarp(GroupMask<L>()); }  // the group has read the row
+		if (grp.leader) { StoreMleRow(row, -1, mp, cd, t, crlb, dev, r.ux, r.uy, ok); }
 	}
-	if (mp.evals && evals) { atomicAdd(mp.evals + 2, evals); }
+	if (mp.evals && evals && grp.leader) { atomicAdd(mp.evals + 2, evals); }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1404,6 +1505,9 @@ int PersistentBlocks(K kernel, size_t smemBytes, int sms, uint32_t cap)
 	return static_cast<int>(std::min<uint32_t>((std::max<uint32_t>(cap, 1) + kThreads - 1) / kThreads, static_cast<uint32_t>(sms * perSm)));
 }
 
+// Lanes per ROI of the FP64 pass (MleFinalKernel has the measurements).
+template <int MODEL> struct FinalLanes { static constexpr int value = MODEL == 8 ? 8 : 1; };
+
 // The four-launch pipeline; the LM and polish run with L lanes per ROI (1: a thread per ROI; 2-16: lane groups).
 template <int MODEL, int L>
 bool LaunchPipeline(const FitImages& fi, const Cand* cands, const uint32_t* nptr, uint32_t nconst,
@@ -1411,23 +1515,31 @@ bool LaunchPipeline(const FitImages& fi, const Cand* cands, const uint32_t* nptr
 {
 	const int sms = SmCount();
 	const uint32_t blocks = std::min<uint32_t>((std::max<uint32_t>(cap, 1) + kThreads - 1) / kThreads, static_cast<uint32_t>(sms) * 32u);
-	const size_t initBytes = static_cast<size_t>(mp.roi) * sizeof(float) * kThreads;
 	const size_t slots = L == 1 ? kThreads : kThreads / L;
 	const size_t lmBytes = static_cast<size_t>(SlotFloats(mp.n, mp.roi, 3, L)) * sizeof(float) * slots;
 	const size_t polishBytes = static_cast<size_t>(SlotFloats(mp.n, mp.roi, 6, L)) * sizeof(float) * slots;
-	const size_t finalBytes = static_cast<size_t>(3 * mp.roi) * sizeof(double) * kThreads;
+	constexpr int FL = FinalLanes<MODEL>::value;
+	const size_t finalBytes = MODEL == 8 ? 0 : static_cast<size_t>((FL == 1 ? 3 : 6) * mp.roi) * sizeof(double) * (kThreads / FL);
+	const uint32_t finalBlocks = static_cast<uint32_t>(std::min<unsigned long long>(
+		(std::max<unsigned long long>(cap, 1) * FL + kThreads - 1) / kThreads, static_cast<unsigned long long>(sms) * 32u));
 	const uint32_t rois = static_cast<uint32_t>(std::min<unsigned long long>(static_cast<unsigned long long>(cap) * L, 0xffffffffull));
 	const int lmBlocks = PersistentBlocks(MleLmKernel<MODEL, L>, lmBytes, sms, rois);
 	const int polishBlocks = PersistentBlocks(MlePolishKernel<MODEL, L>, polishBytes, sms, rois);
 	if (mp.queue && !PTB_CUDA(cudaMemsetAsync(mp.queue, 0, 2 * sizeof(unsigned int), st))) { return false; }
 	if (marks) { cudaEventRecord(marks[0], st); }
-	MleInitKernel<MODEL><<<blocks, kThreads, initBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
+	if constexpr (MODEL == 6) { MleInitKernel<<<blocks, kThreads, 0, st>>>(fi, cands, nptr, nconst, mp, rows); }
+	else {
+		const size_t scanBytes = static_cast<size_t>(ScanSharedWords(mp.n, mp.roi, MODEL)) * sizeof(float);
+		AllowSmem(MleScanKernel<MODEL>, scanBytes);
+		const uint32_t scanBlocks = std::min<uint32_t>((std::max<uint32_t>(cap, 1) - 1) / 32 + 1, static_cast<uint32_t>(sms) * 32u);
+		MleScanKernel<MODEL><<<scanBlocks, 32 * kScanWarps, scanBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
+	}
 	if (marks) { cudaEventRecord(marks[1], st); }
 	MleLmKernel<MODEL, L><<<lmBlocks, kThreads, lmBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
 	if (marks) { cudaEventRecord(marks[2], st); }
 	MlePolishKernel<MODEL, L><<<polishBlocks, kThreads, polishBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
 	if (marks) { cudaEventRecord(marks[3], st); }
-	MleFinalKernel<MODEL><<<blocks, kThreads, finalBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
+	MleFinalKernel<MODEL, FL><<<finalBlocks, kThreads, finalBytes, st>>>(fi, cands, nptr, nconst, mp, rows);
 	if (marks) { cudaEventRecord(marks[4], st); }
 	CountLaunch(4);
 	return PTB_LAUNCHED();

@@ -389,11 +389,11 @@ __global__ void __launch_bounds__(32 * kWarps, 3) SplineFitKernel(const uint16_t
 	}
 }
 
-// The table as given, [64][cells], in the layout the maximum-likelihood spline fit reads, [cells][64] in
-// FP64 and FP32: a tile of 32 cells per CTA, read along the cells and written along the coefficients.
+// The table as given, [64][cells], in the layouts the maximum-likelihood spline fit reads: [cells][64] in FP32 and
+// [16][cells][4] in FP32 and FP64. A tile of 32 cells per CTA, read along the cells and written along the coefficients.
 constexpr int kTableCells = 32;
-__global__ void __launch_bounds__(256) CellTable(const double* __restrict__ given, double* __restrict__ cells64,
-                                                 float* __restrict__ cells32, size_t cells)
+__global__ void __launch_bounds__(256) CellTable(const double* __restrict__ given, double2* __restrict__ quads64,
+                                                 float* __restrict__ cells32, float4* __restrict__ quads32, size_t cells)
 {
 	__shared__ double tile[64][kTableCells + 1];
 	const size_t c0 = static_cast<size_t>(blockIdx.x) * kTableCells;
@@ -404,9 +404,17 @@ __global__ void __launch_bounds__(256) CellTable(const double* __restrict__ give
 	__syncthreads();
 	for (int i = threadIdx.x; i < 64 * kTableCells; i += 256) {
 		const int c = i / 64, k = i % 64;
+		if (c0 + c < cells) { cells32[(c0 + c) * 64 + k] = static_cast<float>(tile[k][c]); }
+	}
+	for (int i = threadIdx.x; i < 16 * kTableCells; i += 256) {
+		const int q = i / kTableCells, c = i % kTableCells;
 		if (c0 + c < cells) {
-			cells64[(c0 + c) * 64 + k] = tile[k][c];
-			cells32[(c0 + c) * 64 + k] = static_cast<float>(tile[k][c]);
+			const double v[4] = {tile[4 * q][c], tile[4 * q + 1][c], tile[4 * q + 2][c], tile[4 * q + 3][c]};
+			double2* at = quads64 + (q * cells + c0 + c) * 2;
+			at[0] = make_double2(v[0], v[1]);
+			at[1] = make_double2(v[2], v[3]);
+			quads32[q * cells + c0 + c] = make_float4(static_cast<float>(v[0]), static_cast<float>(v[1]), static_cast<float>(v[2]),
+			                                          static_cast<float>(v[3]));
 		}
 	}
 }
@@ -423,9 +431,10 @@ __global__ void SwapTable(const double* __restrict__ given, double* __restrict__
 
 }  // namespace
 
-bool LaunchCellTable(const double* given, double* cells64, float* cells32, size_t cells, cudaStream_t st)
+bool LaunchCellTable(const double* given, double* quads64, float* cells32, float* quads32, size_t cells, cudaStream_t st)
 {
-	CellTable<<<static_cast<unsigned>((cells + kTableCells - 1) / kTableCells), 256, 0, st>>>(given, cells64, cells32, cells);
+	CellTable<<<static_cast<unsigned>((cells + kTableCells - 1) / kTableCells), 256, 0, st>>>(
+		given, reinterpret_cast<double2*>(quads64), cells32, reinterpret_cast<float4*>(quads32), cells);
 	CountLaunch();
 	return PTB_LAUNCHED();
 }

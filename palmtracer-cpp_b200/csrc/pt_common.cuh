@@ -190,8 +190,10 @@ struct MleParams {
 	double astig[10];
 	int sx, sy, sz;
 	double dz;
-	const float* table;        // mode 8: cell-major [cell][64], FP32 (FP32 phases)
-	const double* table64;     // mode 8: the same in FP64 (FP64 phases)
+	long long cells;           // mode 8: sx * sy * sz
+	const float* table;        // mode 8: cell-major [cell][64], FP32 (FP32 phases, a thread per ROI)
+	const float* tableQ;       // mode 8: [16][cell][4], FP32 (FP32 phases, lane groups)
+	const double* table64;     // mode 8: [16][cell][4], FP64 (FP64 phases)
 	unsigned int* fallbacks;   // FP64 Cholesky re-factorisations (diagnostics)
 	unsigned int* queue;       // 2 work-queue counters of the persistent fit kernels (zeroed by the launch), or null;
 	                           // modes 1-4 use the first

@@ -334,8 +334,16 @@ bool Pageable(const void* p)
 bool Engine::RingReady()
 {
 	for (int i = 0; i < kRing; ++i) {
-		if (!ring_[i] && !PTB_CUDA(cudaMallocHost(&ring_[i], kRingBytes))) { return false; }
-		if (!ringEv_[i] && !PTB_CUDA(cudaEventCreateWithFlags(&ringEv_[i], cudaEventDisableTiming))) { return false; }
+		if (!ring_[i] && cudaMallocHost(&ring_[i], kRingBytes) != cudaSuccess) {
+			ring_[i] = nullptr;
+			cudaGetLastError();  // not an error of the call: its copies do without the ring
+			return false;
+		}
+		if (!ringEv_[i] && cudaEventCreateWithFlags(&ringEv_[i], cudaEventDisableTiming) != cudaSuccess) {
+			ringEv_[i] = nullptr;
+			cudaGetLastError();
+			return false;
+		}
 	}
 	return true;
 }
@@ -343,8 +351,7 @@ bool Engine::RingReady()
 bool Engine::CopyIn(void* device, const void* host, size_t bytes, cudaStream_t st)
 {
 	if (bytes == 0) { return true; }
-	if (!Pageable(host)) { return PTB_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, st)); }
-	if (!RingReady()) { return false; }
+	if (!Pageable(host) || !RingReady()) { return PTB_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, st)); }
 	// a short copy in a few pieces too: the link starts with the first
 	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));
 	for (size_t at = 0; at < bytes; at += piece) {
@@ -363,10 +370,9 @@ bool Engine::CopyIn(void* device, const void* host, size_t bytes, cudaStream_t s
 bool Engine::CopyOut(void* host, const void* device, size_t bytes, cudaStream_t st)
 {
 	if (bytes == 0) { return true; }
-	if (!Pageable(host)) {
+	if (!Pageable(host) || !RingReady()) {
 		return PTB_CUDA(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, st)) && PTB_CUDA(cudaStreamSynchronize(st));
 	}
-	if (!RingReady()) { return false; }
 	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));
 	const uint64_t pieces = (bytes + piece - 1) / piece, first = ringNext_;
 	ringNext_ += pieces;

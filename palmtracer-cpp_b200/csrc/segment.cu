@@ -5,11 +5,11 @@
 //   1. union-find connected components of the domain (8-connectivity) over the sparse domain list;
 //   2. each seed (local maximum) inherits the label of its first raster-earlier seed neighbour, as getLocalMax()
 //      does (Segmentation2D.cpp:309-327); root seeds are numbered in raster order through a per-row bitmask rank;
-//   3. a component with one label is labelled directly; every other component (a "group") is flooded by one thread
-//      (lane 0 of a warp that stages the group's box in shared memory; in strict mode a thread on global memory)
-//      with a binary heap whose push/pop steps are those of libstdc++'s std::priority_queue, with the reference key
-//      -v + pops * 1e-7 (Segmentation2D.cpp:336-385) and a pop counter local to the group. In strict mode a group is
-//      a whole frame and the counter is frame-global, which is the reference's process exactly;
+//   3. a component with one label is labelled directly; every other component (a "group") is flooded by a warp that
+//      stages the group's box in shared memory, with the reference key -v + pops * 1e-7 (Segmentation2D.cpp:336-385),
+//      a pop counter local to the group and, where keys tie, a binary heap whose push/pop steps are those of
+//      libstdc++'s std::priority_queue. In strict mode a group is a whole frame and the counter is frame-global, which
+//      is the reference's process exactly;
 //   4. basin fusion (Segmentation2D.cpp:181-291) per group, then a second flood from one seed per basin;
 //   5. exactness check of every per-component flood (below): a first test per boundary pair, then the rank test of
 //      the pairs that fail it; a frame that fails both is flooded again per component with estimated frame-wide

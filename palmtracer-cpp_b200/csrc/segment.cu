@@ -935,8 +935,9 @@ __device__ bool FloodWarp(Smem& sm, const Geometry& geo, int bx0, int by0, int b
 		const int r = static_cast<int>(p >> 16), c = static_cast<int>(p & 0xffffu), i = r * bw + c;
 		const int rr = r + dr, cc = c + dc, j = rr * bw + cc;
 		const bool push = lane < 8 && rr >= 0 && rr < bh && cc >= 0 && cc < bw && (sm.flag[j] & 1u) && sm.lab[j] == 0;
-		const unsigned m = __ballot_sync(0xffffffffu, push);  // every lane has read what the stores below replace
+		const unsigned m = __ballot_sync(0xffffffffu, push);
 		if (len + __popc(m) > kBoxHeap) { return false; }
+		__syncwarp();  // every lane has read what the stores below replace (votes and shuffles order no memory)
 		if (lane == 31 && e != len) {
 			keys[e] = lastKey;
 			at[e] = lastAt;

@@ -52,6 +52,7 @@ bool CheckCuda(cudaError_t e, const char* what, const char* file, int line)
 {
 	if (e == cudaSuccess) { return true; }
 	SetError(std::string(what) + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")");
+	cudaGetLastError();  // reported: the thread's next launch check must not find it again
 	return false;
 }
 

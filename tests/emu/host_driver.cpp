@@ -1,0 +1,46 @@
+// The library's host code on the stand-in runtime (fake_cudart.cpp), one check per name on the command line. A check
+// prints what it saw and the driver returns 0 when all hold. Test harness only.
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "../../include/palmtracer_b200.h"
+#include "fake_cudart.h"
+
+namespace {
+
+int failures = 0;
+
+void Expect(bool ok, const char* what)
+{
+	std::printf("%s %s (%s)\n", ok ? "ok  " : "FAIL", what, PTB_LastError());
+	failures += ok ? 0 : 1;
+}
+
+const double kParams[4] = {7, 1, 2, 0};
+
+// A call that was refused (here: no device memory) is over: the next one does not fail for it.
+void AfterAnError()
+{
+	const uint64_t H = 64, W = 80, Z = 3, n = 5;
+	std::vector<uint16_t> stack(2 * H * W * Z, 100);
+	std::vector<double> pos(n * 6, 1.0), rows(n * 18);
+	auto fit = [&](uint64_t planes) { return Fitting(stack.data(), pos.data(), n, rows.data(), rows.size(), H, W, planes, 2, kParams); };
+	Expect(fit(Z) == n * 18, "Fitting");
+	const size_t had = fake::limit;
+	fake::limit = 0;
+	Expect(fit(2 * Z) == 0 && *PTB_LastError(), "Fitting without device memory");
+	fake::limit = had;
+	Expect(fit(Z) == n * 18, "Fitting afterwards");
+}
+
+}  // namespace
+
+int main(int argc, char** argv)
+{
+	for (int i = 1; i < argc; ++i) {
+		if (!std::strcmp(argv[i], "after")) { AfterAnError(); }
+		else { return 2; }
+	}
+	return failures ? 1 : 0;
+}

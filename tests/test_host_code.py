@@ -1,0 +1,13 @@
+"""The library's host code without a GPU: its objects run on a stand-in for the CUDA runtime (tests/emu/fake_cudart.cpp)
+whose device memory is host memory and whose kernels do nothing."""
+import hostcode
+import pytest
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    return hostcode.link(tmp_path_factory.mktemp("host") / "host", ["host_driver.cpp"])
+
+
+def test_a_call_after_a_refused_call(driver):
+    assert hostcode.run(driver, "after") == 0

@@ -352,7 +352,9 @@ bool Engine::RingReady()
 bool Engine::CopyIn(void* device, const void* host, size_t bytes, cudaStream_t st)
 {
 	if (bytes == 0) { return true; }
-	if (!Pageable(host) || !RingReady()) { return PTB_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, st)); }
+	if (!host || !Pageable(host) || !RingReady()) {  // a null buffer is the runtime's error
+		return PTB_CUDA(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, st));
+	}
 	// a short copy in a few pieces too: the link starts with the first
 	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));
 	for (size_t at = 0; at < bytes; at += piece) {
@@ -371,7 +373,7 @@ bool Engine::CopyIn(void* device, const void* host, size_t bytes, cudaStream_t s
 bool Engine::CopyOut(void* host, const void* device, size_t bytes, cudaStream_t st)
 {
 	if (bytes == 0) { return true; }
-	if (!Pageable(host) || !RingReady()) {
+	if (!host || !Pageable(host) || !RingReady()) {
 		return PTB_CUDA(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, st)) && PTB_CUDA(cudaStreamSynchronize(st));
 	}
 	const size_t piece = std::min(kRingBytes, std::max<size_t>(1 << 20, bytes / kRing));

@@ -34,12 +34,32 @@ void AfterAnError()
 	Expect(fit(Z) == n * 18, "Fitting afterwards");
 }
 
+// Null buffers are refused with the runtime's error by every entry point that hands host memory to a copy.
+void NullBuffers()
+{
+	const uint64_t H = 64, W = 80, Z = 3, n = 5;
+	std::vector<uint16_t> stack(H * W * Z, 100);
+	std::vector<double> pos(n * 6, 1.0), rows(n * 18), plane(H * W * Z), points(n * 4, 1.0);
+	std::vector<uint64_t> tracks(n * 2);
+	Expect(Fitting(nullptr, pos.data(), n, rows.data(), rows.size(), H, W, Z, 2, kParams) == 0 && *PTB_LastError(), "Fitting of a null stack");
+	Expect(Fitting(stack.data(), pos.data(), n, nullptr, rows.size(), H, W, Z, 2, kParams) == 0 && *PTB_LastError(), "Fitting into a null buffer");
+	Wavelett(nullptr, plane.data(), H, W, Z, 2);
+	Expect(*PTB_LastError(), "Wavelett of a null stack");
+	Wavelett(stack.data(), nullptr, H, W, Z, 2);
+	Expect(*PTB_LastError(), "Wavelett into a null buffer");
+	Tracking(nullptr, tracks.data(), n, 5.0);
+	Expect(*PTB_LastError(), "Tracking of a null table");
+	Expect(Localization(nullptr, rows.data(), rows.size(), H, W, Z, 10.0, 0.0, 0, kParams) == 0 && *PTB_LastError(), "Localization of a null stack");
+	Expect(Fitting(stack.data(), pos.data(), n, rows.data(), rows.size(), H, W, Z, 2, kParams) == n * 18, "Fitting afterwards");
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
 {
 	for (int i = 1; i < argc; ++i) {
 		if (!std::strcmp(argv[i], "after")) { AfterAnError(); }
+		else if (!std::strcmp(argv[i], "null")) { NullBuffers(); }
 		else { return 2; }
 	}
 	return failures ? 1 : 0;

@@ -11,3 +11,9 @@ def driver(tmp_path_factory):
 
 def test_a_call_after_a_refused_call(driver):
     assert hostcode.run(driver, "after") == 0
+
+
+def test_null_buffers_are_refused(driver):
+    """A null stack, table or output is an error of the call, as the runtime reports it, for the entry points whose
+    pageable copies go through the pinned ring too."""
+    assert hostcode.run(driver, "null") == 0

@@ -6,6 +6,8 @@
 // capacity can overflow; the budget only bounds B.
 #include "engine.h"
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -206,10 +208,20 @@ namespace {
 // caller waits for the last tasks without sleeping: waking either takes longer than a job.
 class CopyThreads {
 public:
+	// Ended at exit by the process that started them: a forked child has none of the threads, and must neither join them
+	// nor take down what they wait on.
 	static CopyThreads& Get()
 	{
-		static CopyThreads t;
-		return t;
+		struct Owner {
+			CopyThreads* const threads = new CopyThreads;
+			const pid_t process = getpid();
+			~Owner()
+			{
+				if (getpid() == process) { delete threads; }
+			}
+		};
+		static Owner owner;
+		return *owner.threads;
 	}
 
 	// Calls task(0) .. task(n - 1) on the helpers and the calling thread; returns when all have finished.

@@ -1,11 +1,21 @@
 // The library's host code on the stand-in runtime (fake_cudart.cpp), one check per name on the command line. A check
 // prints what it saw and the driver returns 0 when all hold. Test harness only.
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
+#include <signal.h>
+#include <sys/wait.h>
+#include <time.h>
+#include <unistd.h>
+
 #include "../../include/palmtracer_b200.h"
 #include "fake_cudart.h"
+
+namespace ptb {
+void ParallelCopy(void* dst, const void* src, size_t bytes);
+}
 
 namespace {
 
@@ -53,6 +63,23 @@ void NullBuffers()
 	Expect(Fitting(stack.data(), pos.data(), n, rows.data(), rows.size(), H, W, Z, 2, kParams) == n * 18, "Fitting afterwards");
 }
 
+// A child forked from a process whose copies have helper threads exits with its own code: it has none of the threads.
+void ForkedChild()
+{
+	std::vector<char> from(8 << 20, 7), to(from.size());
+	ptb::ParallelCopy(to.data(), from.data(), from.size());
+	const timespec pause{0, 20000000};
+	nanosleep(&pause, nullptr);  // the helpers have gone to sleep
+	std::fflush(stdout);
+	const pid_t child = fork();
+	if (child == 0) { std::exit(7); }
+	int status = 0, seen = 0;
+	for (int i = 0; i < 500 && (seen = waitpid(child, &status, WNOHANG)) == 0; ++i) { nanosleep(&pause, nullptr); }
+	if (seen == 0) { kill(child, SIGKILL); }
+	Expect(to == from, "the copy");
+	Expect(seen == child && WIFEXITED(status) && WEXITSTATUS(status) == 7, "exit of a forked child");
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -60,6 +87,7 @@ int main(int argc, char** argv)
 	for (int i = 1; i < argc; ++i) {
 		if (!std::strcmp(argv[i], "after")) { AfterAnError(); }
 		else if (!std::strcmp(argv[i], "null")) { NullBuffers(); }
+		else if (!std::strcmp(argv[i], "fork")) { ForkedChild(); }
 		else { return 2; }
 	}
 	return failures ? 1 : 0;

@@ -17,3 +17,8 @@ def test_null_buffers_are_refused(driver):
     """A null stack, table or output is an error of the call, as the runtime reports it, for the entry points whose
     pageable copies go through the pinned ring too."""
     assert hostcode.run(driver, "null") == 0
+
+
+def test_forked_child_exits(driver):
+    """A child process forked after the library has copied with helper threads ends with its own exit code."""
+    assert hostcode.run(driver, "fork") == 0

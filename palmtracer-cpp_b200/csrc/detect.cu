@@ -529,15 +529,11 @@ __global__ void __launch_bounds__(kThreads) PlaneKernel(const uint16_t* __restri
 	}
 }
 
-// Once per process (a function-local static is initialised once, also when several threads call at the same time).
 bool ConfigureSmem()
 {
-	static const bool done = [] {
-		const int bytes = static_cast<int>(sizeof(TileSmem));
-		bool ok = PTB_CUDA(cudaFuncSetAttribute(DetectKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDetectBytes));
-		return ok && PTB_CUDA(cudaFuncSetAttribute(PlaneKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-	}();
-	return done;
+	static std::atomic<uint64_t> detect{0}, plane{0};
+	return AllowSmemOnDevice(reinterpret_cast<const void*>(DetectKernel), kDetectBytes, detect) &&
+	       AllowSmemOnDevice(reinterpret_cast<const void*>(PlaneKernel), sizeof(TileSmem), plane);
 }
 
 // The driver's tensor-map encoder (cuTensorMapEncodeTiled), fetched once through the runtime so that the library

@@ -174,6 +174,17 @@ uint32_t IndepBound(int H, int W) { return static_cast<uint32_t>(((H + 1) / 2)) 
 
 }  // namespace
 
+bool AllowSmemOnDevice(const void* kernel, size_t bytes, std::atomic<uint64_t>& devices)
+{
+	int dev = 0;
+	if (!PTB_CUDA(cudaGetDevice(&dev))) { return false; }
+	const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+	if (devices.load(std::memory_order_relaxed) & bit) { return true; }
+	if (!PTB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)))) { return false; }
+	devices.fetch_or(bit, std::memory_order_relaxed);
+	return true;
+}
+
 cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
 {
 	constexpr int kDevices = 64;

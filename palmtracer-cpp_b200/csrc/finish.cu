@@ -269,9 +269,8 @@ bool LaunchBuildCandidates(const Workspace& ws, cudaStream_t st)
 bool LaunchSortFrames(const Workspace& ws, double* out, unsigned long long* rowBase, bool offsetOut, unsigned long long planeBase,
                       cudaStream_t st)
 {
-	static const bool configured = PTB_CUDA(cudaFuncSetAttribute(SortFrames, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                                             static_cast<int>(kSortSmemBytes)));
-	if (!configured) { return false; }
+	static std::atomic<uint64_t> devices{0};
+	if (!AllowSmemOnDevice(reinterpret_cast<const void*>(SortFrames), kSortSmemBytes, devices)) { return false; }
 	// with few frames several CTAs order and write each of them, up to the number of SMs (BandOrder has the measurements)
 	const int parts = std::max(1, std::min(16, 148 / std::max(1, ws.g.B)));
 	SortFrames<<<dim3(ws.g.B, parts), kSortThreads, kSortSmemBytes, st>>>(ws, out, rowBase, offsetOut ? 1 : 0, planeBase, ws.capRows);

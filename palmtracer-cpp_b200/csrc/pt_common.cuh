@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
@@ -70,6 +71,10 @@ void CountLaunch(uint64_t n = 1);
 // 396 000 points on the device: 1.53 ms, with this pool 0.46 ms).
 constexpr size_t kScratchKeep = 1ull << 30;
 cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st);
+
+// Allows a kernel `bytes` of dynamic shared memory on the current device, where the runtime keeps that setting: asked for
+// once per device (`devices`, a static of the launch: the devices that have it).
+bool AllowSmemOnDevice(const void* kernel, size_t bytes, std::atomic<uint64_t>& devices);
 
 #define PTB_CUDA(call) ::ptb::CheckCuda((call), #call, __FILE__, __LINE__)
 #define PTB_LAUNCHED() ::ptb::CheckCuda(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)

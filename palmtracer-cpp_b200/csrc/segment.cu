@@ -2586,9 +2586,9 @@ bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPo
 	}
 	// frame-wide groups: a warp per frame
 	auto frameFlood = [&](int routed) {
-		static const bool heapSmem = PTB_CUDA(cudaFuncSetAttribute(FrameFlood, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                                                           static_cast<int>(kFrameHeapBytes)));
-		ok = ok && heapSmem && LaunchChained(FrameFlood, static_cast<int>(std::min<uint32_t>(frames, 148u)), 32, kFrameHeapBytes, st, ws, routed);
+		static std::atomic<uint64_t> devices{0};
+		ok = ok && AllowSmemOnDevice(reinterpret_cast<const void*>(FrameFlood), kFrameHeapBytes, devices) &&
+		     LaunchChained(FrameFlood, static_cast<int>(std::min<uint32_t>(frames, 148u)), 32, kFrameHeapBytes, st, ws, routed);
 		CountLaunch();
 	};
 	launch(GroupScatter, grid, kThreads, strict ? 1 : 0);
@@ -2606,9 +2606,9 @@ bool LaunchSegment(const Workspace& ws, double ratio, int strict, uint32_t maxPo
 		launch(SuspectCheck, std::min(grid, 64), kThreads, 0);
 		launch(RefloodPlan, 1, kPlanThreads);
 		launch(RefloodGather, grid, kThreads);
-		static const bool bucketSmem = PTB_CUDA(cudaFuncSetAttribute(RefloodBucket, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                                                             static_cast<int>(kRfBucketSmem)));
-		ok = ok && bucketSmem && LaunchChained(RefloodBucket, RefloodSlots(g) * 2, kRfBucketThreads, kRfBucketSmem, st, ws);
+		static std::atomic<uint64_t> devices{0};
+		ok = ok && AllowSmemOnDevice(reinterpret_cast<const void*>(RefloodBucket), kRfBucketSmem, devices) &&
+		     LaunchChained(RefloodBucket, RefloodSlots(g) * 2, kRfBucketThreads, kRfBucketSmem, st, ws);
 		CountLaunch();
 		launch(RefloodCounts, grid, kThreads);
 		launch(RefloodBox, grid, kRfWarps * 32);

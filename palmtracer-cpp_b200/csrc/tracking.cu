@@ -373,9 +373,8 @@ constexpr size_t kSegSmemBytes = 2 * kSegSmem * sizeof(unsigned long long);
 bool LaunchSegmentSort(unsigned long long* k1, unsigned long long* k2, const uint32_t* off, uint32_t nseg, unsigned long long* s1,
                        unsigned long long* s2, cudaStream_t st, const uint32_t* pending = nullptr)
 {
-	static const bool configured = PTB_CUDA(cudaFuncSetAttribute(SegmentSort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                                             static_cast<int>(kSegSmemBytes)));
-	if (!configured) { return false; }
+	static std::atomic<uint64_t> devices{0};
+	if (!AllowSmemOnDevice(reinterpret_cast<const void*>(SegmentSort), kSegSmemBytes, devices)) { return false; }
 	SegmentSort<<<std::max<uint32_t>(1, std::min<uint32_t>(nseg, 148u * 32)), kSortThreads, kSegSmemBytes, st>>>(k1, k2, off, nseg, s1, s2, pending);
 	CountLaunch();
 	return PTB_LAUNCHED();

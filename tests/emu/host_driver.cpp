@@ -10,6 +10,8 @@
 #include <time.h>
 #include <unistd.h>
 
+#include <cuda_runtime_api.h>
+
 #include "../../include/palmtracer_b200.h"
 #include "fake_cudart.h"
 
@@ -80,6 +82,27 @@ void ForkedChild()
 	Expect(seen == child && WIFEXITED(status) && WEXITSTATUS(status) == 7, "exit of a forked child");
 }
 
+// Every entry point on a second device after the first: kernels are allowed their shared memory on each.
+void SecondDevice()
+{
+	const uint64_t H = 64, W = 80, Z = 3, n = 5;
+	std::vector<uint16_t> stack(H * W * Z, 100);
+	std::vector<double> pos(n * 6, 1.0), rows(n * 18 * Z), plane(H * W * Z);
+	for (int device = 0; device < fake::kDevices; ++device) {
+		cudaSetDevice(device);
+		const size_t before = fake::launches[device];
+		Localization(stack.data(), rows.data(), rows.size(), H, W, Z, 10.0, 10.0, 2, kParams);
+		Expect(!*PTB_LastError() && fake::launches[device] > before, device ? "Localization on device 1" : "Localization on device 0");
+		const int mode = PTB_SetSegmentationMode(1);
+		Localization(stack.data(), rows.data(), rows.size(), H, W, Z, 10.0, 10.0, 0, kParams);
+		Expect(!*PTB_LastError(), device ? "strict segmentation on device 1" : "strict segmentation on device 0");
+		PTB_SetSegmentationMode(mode);
+		Wavelett(stack.data(), plane.data(), H, W, Z, 2);
+		Expect(!*PTB_LastError(), device ? "Wavelett on device 1" : "Wavelett on device 0");
+	}
+	cudaSetDevice(0);
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -88,6 +111,7 @@ int main(int argc, char** argv)
 		if (!std::strcmp(argv[i], "after")) { AfterAnError(); }
 		else if (!std::strcmp(argv[i], "null")) { NullBuffers(); }
 		else if (!std::strcmp(argv[i], "fork")) { ForkedChild(); }
+		else if (!std::strcmp(argv[i], "devices")) { SecondDevice(); }
 		else { return 2; }
 	}
 	return failures ? 1 : 0;

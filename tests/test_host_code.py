@@ -22,3 +22,9 @@ def test_null_buffers_are_refused(driver):
 def test_forked_child_exits(driver):
     """A child process forked after the library has copied with helper threads ends with its own exit code."""
     assert hostcode.run(driver, "fork") == 0
+
+
+def test_second_device(driver):
+    """A process that calls the library with one device current and then with another: the kernels that take more than
+    48 KB of shared memory are allowed it on both."""
+    assert hostcode.run(driver, "devices") == 0

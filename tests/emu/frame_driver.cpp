@@ -2,7 +2,8 @@
 // launch order: per-component floods with both exactness tests and the re-flood, basin fusion, the frame-wide flood by a
 // warp, region sums and the frames' offsets, with the library's prefix sums. Every device array is a separate
 // allocation for AddressSanitizer. Test harness only.
-// Usage: frame_emu <in> <out> [warps]; in: int32 H, W, B, mode, int64 threshold (2^-16 units), double fusion ratio,
+// Usage: frame_emu order <seeds> <pixels> <first pixel> checks and times the order of a frame's seeds;
+// frame_emu <in> <out> [warps]; in: int32 H, W, B, mode, int64 threshold (2^-16 units), double fusion ratio,
 // B * H * W int64 W1 values (2^-16 units); warps: warps per block of the kernels that give a warp a group (0: as the
 // library). out: B * H * W uint32 labels, B * H * W code bytes, B + 1 uint32 output offsets, then 7 uint32 (routed,
 // rank-tested, re-flooded, groups fused in global memory, fits, fault, multi-label groups).
@@ -23,6 +24,7 @@ thread_local uint32_t collectives;
 #include "scan_emu.inc"
 #include "frame_emu.inc"
 
+#include <chrono>
 #include <cstdio>
 #include <cstdlib>
 
@@ -71,10 +73,39 @@ void Scan(std::initializer_list<ScanJob> jobs, unsigned* fault)
 	for (auto* p : states) { free(p); }
 }
 
+void OrderKernel(const uint32_t* seeds, uint32_t n, uint32_t base, unsigned long long N, uint32_t* sorted)
+{
+	static uint32_t count[kSeedBuckets];
+	OrderSeeds(seeds, n, base, N, sorted, count);
+}
+
+// `n` seeds of a frame of N pixels that starts at pixel `base`, in the order of a fixed shuffle: 0 when they come out
+// ascending. Prints the milliseconds it took.
+int OrderCheck(uint32_t n, unsigned long long N, uint32_t base)
+{
+	std::vector<uint32_t> want(n);
+	for (uint32_t i = 0; i < n; ++i) { want[i] = base + static_cast<uint32_t>(i * N / n); }  // distinct for n <= N
+	uint32_t* seeds = Alloc<uint32_t>(n);
+	uint32_t* sorted = Alloc<uint32_t>(n);
+	std::copy(want.begin(), want.end(), seeds);
+	unsigned long long r = 88172645463325252ull;
+	for (uint32_t i = n; i > 1; --i) {
+		r ^= r << 13; r ^= r >> 7; r ^= r << 17;
+		std::swap(seeds[i - 1], seeds[r % i]);
+	}
+	const auto t0 = std::chrono::steady_clock::now();
+	Run(dim3(1), 32, OrderKernel, static_cast<const uint32_t*>(seeds), n, base, N, sorted);
+	printf("%.3f\n", std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+	return std::equal(want.begin(), want.end(), sorted) ? 0 : 1;
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
 {
+	if (argc == 5 && !strcmp(argv[1], "order")) {
+		return OrderCheck(static_cast<uint32_t>(atoll(argv[2])), static_cast<unsigned long long>(atoll(argv[3])), static_cast<uint32_t>(atoll(argv[4])));
+	}
 	if (argc < 3) { return 2; }
 	const int warps = argc > 3 ? atoi(argv[3]) : 0;
 	FILE* fp = fopen(argv[1], "rb");

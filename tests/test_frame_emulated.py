@@ -107,3 +107,28 @@ def test_box_flood_orders_its_accesses(racecheck, orc):
     print(stats, "label differences", diff)
     assert diff == 0 and stats["groups"] >= 3, stats
     assert _reports(err, "FloodWarp") == [], _reports(err, "FloodWarp")[0][:3000]
+
+
+@pytest.fixture(scope="module")
+def boundscheck(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("frame_asan"), "address")
+
+
+def _order(exe, n, pixels, base):
+    r = subprocess.run([str(exe), "order", str(n), str(pixels), str(base)], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, (n, pixels, base, r.stderr[-2000:])
+    return float(r.stdout)
+
+
+@pytest.mark.parametrize("n, pixels, base", [(0, 100, 0), (1, 1, 7), (31, 31, 5), (33, 100, 200), (4000, 4000, 12345), (9000, 32768, 0),
+                                             (5000, 32769, 2 * 32769), (20000, 1 << 20, 1 << 30), (3000, 2147483647, 0)])
+def test_seed_order(boundscheck, n, pixels, base):
+    """A frame's seeds in raster order: fewer pixels than bands, as many, one more, and the largest frame."""
+    _order(boundscheck, n, pixels, base)
+
+
+def test_seed_order_grows_with_the_seeds(boundscheck):
+    """Sixteen times the seeds take about sixteen times as long (comparing all with all took 256 times)."""
+    small, large = (min(_order(boundscheck, n, 1 << 22, 0) for _ in range(3)) for n in (1 << 15, 1 << 19))
+    print("ms", small, large)
+    assert large < 64 * small

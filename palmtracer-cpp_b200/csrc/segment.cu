@@ -1574,7 +1574,11 @@ __global__ void __launch_bounds__(kFuseWarps * 32) GroupFuseBox(Workspace ws, do
 
 // Basin fusion of one group (Segmentation2D.cpp:181-291) followed by the reseeded second flood.
 // Groups: the per-component groups that GroupFuseBox listed (nGroupsStrict = 0; the second flood is checked for
-// exactness), every frame (strict mode) or only the frames flooded again frame-wide (routed).
+// exactness), every frame (strict mode) or only the frames flooded again frame-wide (routed). One thread per group, the
+// groups dealt to the CTAs first: neighbours in the list share no SM's issue slots and L1 while others are free. Filling
+// one CTA after the other left 300 frames to five CTAs, which a chained launch sets up on the first SM that has room:
+// 300 strict 256 x 256 frames with fusion took 191 ms (185 with plain launches), dealt this way 48 ms, 64 such frames 120
+// and 34 ms.
 __global__ void __launch_bounds__(kFloodThreads) GroupFuse(Workspace ws, uint32_t nGroupsStrict, double ratio, int routed)
 {
 	PTB_AFTER_PREVIOUS();
@@ -1582,7 +1586,7 @@ __global__ void __launch_bounds__(kFloodThreads) GroupFuse(Workspace ws, uint32_
 	if (routed && ws.cnt->nroute == 0) { return; }
 	const uint32_t n = nGroupsStrict ? nGroupsStrict : ws.cnt->nfuse;
 	const Geometry& geo = ws.g;
-	for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+	for (uint32_t k = threadIdx.x * gridDim.x + blockIdx.x; k < n; k += gridDim.x * blockDim.x) {
 		const uint32_t m = nGroupsStrict ? k : ws.rfGroups[k];
 		if (routed && ws.frameRoute[m] == 0) { continue; }
 		uint32_t* regs = ws.gReg + ws.gRegOff[m];

@@ -964,8 +964,10 @@ __device__ void FloodGroupGlobal(const Workspace& ws, const uint32_t* seedList, 
 	FloodGroup<kChain>(ws.g, GlobalView{ws}, seedList, nSeeds, heap);
 }
 
-// Frame-wide floods by one thread per frame, the steps FrameFlood follows (the CPU emulation runs this form): every
-// frame or only the frames that failed the exactness test of their per-component floods (routed).
+#if !defined(__CUDACC__)
+// Frame-wide floods by one thread per frame, the steps FrameFlood follows: every frame or only the frames that failed the
+// exactness test of their per-component floods (routed). Not part of the library: the CPU emulation of one frame's
+// kernels floods with it.
 __global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32_t nFrames, int routed)
 {
 	PTB_AFTER_PREVIOUS();
@@ -979,6 +981,7 @@ __global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32
 		FloodGroupGlobal<false>(ws, seeds, nSeeds, ws.heapKey + ws.gOff[m], ws.heapPix + ws.gOff[m], sm);
 	}
 }
+#endif
 
 // ---- Frame-wide flood by a warp -----------------------------------------------------------------------------------
 // A whole frame's flood (a routed frame, or every frame in strict mode) with its open entries in a 32-ary heap, its

@@ -1,13 +1,19 @@
-// Runs the segmentation of a chunk of frames on the CPU (each CUDA thread a host thread, warp_shim.h) in the library's
+// Runs the segmentation of a chunk of frames on the CPU (each CUDA thread a host thread) in the library's
 // launch order: per-component floods with both exactness tests and the re-flood, basin fusion, the frame-wide flood by a
 // warp, region sums and the frames' offsets, with the library's prefix sums. Every device array is a separate
 // allocation for AddressSanitizer. Test harness only.
-// Usage: frame_emu order <seeds> <pixels> <first pixel> checks and times the order of a frame's seeds;
-// frame_emu <in> <out> [warps]; in: int32 H, W, B, mode, int64 threshold (2^-16 units), double fusion ratio,
+// Usage: frame_emu order <seeds> <pixels> <first pixel> checks and times the order of a frame's seeds; frame_emu scan
+// <entries> <capacity> <CTAs> and frame_emu lookback <tile> <prefix> <missing> check the prefix sums;
+// frame_emu <in> <out> [warps [points per frame]]; in: int32 H, W, B, mode, int64 threshold (2^-16 units), double fusion ratio,
 // B * H * W int64 W1 values (2^-16 units); warps: warps per block of the kernels that give a warp a group (0: as the
 // library). out: B * H * W uint32 labels, B * H * W code bytes, B + 1 uint32 output offsets, then 7 uint32 (routed,
 // rank-tested, re-flooded, groups fused in global memory, fits, fault, multi-label groups).
+// PTB_UNORDERED: warp collectives that order no memory (for ThreadSanitizer); otherwise on barriers, which is faster.
+#if defined(PTB_UNORDERED)
 #include "warp_shim.h"
+#else
+#include "shim.h"
+#endif
 
 thread_local uint3 threadIdx;
 thread_local uint3 blockIdx;
@@ -17,8 +23,10 @@ namespace emu {
 std::barrier<>* blockBar;
 std::vector<std::unique_ptr<std::barrier<>>> warpBar;
 uint64_t xbuf[1024];
+#if defined(PTB_UNORDERED)
 Slot slots[2][1024];
 thread_local uint32_t collectives;
+#endif
 }  // namespace emu
 
 #include "scan_emu.inc"
@@ -49,9 +57,13 @@ namespace {
 // threads take no value left by another's.
 template <class K, class... A> void Run(dim3 grid, int threads, K kernel, A... args)
 {
+#if defined(PTB_UNORDERED)
 	memset(static_cast<void*>(emu::slots), 0, sizeof emu::slots);
+#endif
 	emu::Launch(grid, dim3(threads), [=]() {
+#if defined(PTB_UNORDERED)
 		emu::collectives = (blockIdx.y * grid.x + blockIdx.x) << 24;
+#endif
 		kernel(args...);
 	});
 }
@@ -99,15 +111,70 @@ int OrderCheck(uint32_t n, unsigned long long N, uint32_t base)
 	return std::equal(want.begin(), want.end(), sorted) ? 0 : 1;
 }
 
+// Prefix sums of n entries counted on the device (capacity cap), by the given number of CTAs: 0 when they are right.
+int ScanCheck(uint32_t n, uint32_t cap, uint32_t blocks)
+{
+	const uint32_t held = std::min(n, cap);
+	uint32_t* data = Alloc<uint32_t>(cap + 1);
+	uint32_t* count = Alloc<uint32_t>(1);
+	unsigned long long* state = Alloc<unsigned long long>(ScanStateWords(cap));
+	std::vector<uint32_t> want(held + 1, 0);
+	for (uint32_t i = 0; i < held; ++i) {
+		data[i] = (i * 2654435761u) >> 20;
+		want[i + 1] = want[i] + data[i];
+	}
+	memset(state, 0, ScanStateWords(cap) * sizeof(unsigned long long));
+	*count = n;
+	Scans s{};
+	uint32_t total = 0, fault = 0;
+	s.job[0] = ScanJob{data, count, 0, cap, &total};
+	s.state[0] = state;
+	s.fault = &fault;
+	Run(dim3(blocks, 1), kScanThreads, ScanKernel, s);
+	return fault == 0 && total == want[held] && std::equal(want.begin(), want.end(), data) ? 0 : 1;
+}
+
+void LookBackKernel(unsigned long long* tiles, uint32_t tile, uint32_t* fault, uint32_t* sum)
+{
+	const uint32_t s = LookBack(tiles, tile, fault);
+	if (threadIdx.x == 0) { *sum = s; }
+}
+
+// The sum before `tile` from its predecessors' states: sums from `prefix` on, where a whole prefix is published (-1:
+// nowhere), and with `missing` (-1: none) not published at all, which the bounded wait has to report.
+int LookBackCheck(uint32_t tile, int prefix, int missing)
+{
+	unsigned long long* tiles = Alloc<unsigned long long>(tile);
+	uint32_t want = 0, fault = 0, sum = 0;
+	for (uint32_t i = 0; i < tile; ++i) {
+		const uint32_t v = 1000 + i * 7;
+		tiles[i] = kSum | v;
+		if (static_cast<int>(i) == prefix) {
+			tiles[i] = kPrefix | 123456u;
+			want = 123456u;
+		}
+		else if (static_cast<int>(i) > prefix) { want += v; }
+	}
+	if (prefix < 0) { tiles[0] = kPrefix | 1000u; }
+	if (missing >= 0) { tiles[missing] = 0; }
+	Run(dim3(1), 32, LookBackKernel, tiles, tile, &fault, &sum);
+	return missing >= 0 ? (fault == 1 ? 0 : 1) : (fault == 0 && sum == want ? 0 : 1);
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
 {
+	if (argc == 5 && !strcmp(argv[1], "scan")) {
+		return ScanCheck(static_cast<uint32_t>(atoll(argv[2])), static_cast<uint32_t>(atoll(argv[3])), static_cast<uint32_t>(atoll(argv[4])));
+	}
+	if (argc == 5 && !strcmp(argv[1], "lookback")) { return LookBackCheck(static_cast<uint32_t>(atoll(argv[2])), atoi(argv[3]), atoi(argv[4])); }
 	if (argc == 5 && !strcmp(argv[1], "order")) {
 		return OrderCheck(static_cast<uint32_t>(atoll(argv[2])), static_cast<unsigned long long>(atoll(argv[3])), static_cast<uint32_t>(atoll(argv[4])));
 	}
 	if (argc < 3) { return 2; }
 	const int warps = argc > 3 ? atoi(argv[3]) : 0;
+	const uint32_t maxPoints = argc > 4 ? static_cast<uint32_t>(atoi(argv[4])) : 0xffffffffu;
 	FILE* fp = fopen(argv[1], "rb");
 	int dims[4] = {};
 	long long thr = 0;
@@ -238,8 +305,8 @@ int main(int argc, char** argv)
 	Run(two, 128, RegionStats, ws);
 	Run(two, 128, CandidateFlags, ws);
 	Scan({{ws.regCand, &ws.cnt->nregion, 0, ws.capRegion, &ws.cnt->ncand}}, &ws.cnt->fault);
-	Run(one, kOffsetThreads, FrameOffsets, ws, ws.capRows);
-	Run(two, 128, CandidateEmit, ws, ws.capRows);
+	Run(one, kOffsetThreads, FrameOffsets, ws, maxPoints);
+	Run(two, 128, CandidateEmit, ws, maxPoints);
 	FILE* lf = fopen(argv[2], "wb");
 	fwrite(ws.lab, sizeof(uint32_t), P, lf);
 	fwrite(ws.code, 1, P, lf);

@@ -1,6 +1,7 @@
 // shim.h with warp collectives that order no memory, as the hardware's: a ballot or shuffle hands over values only, and
 // between lanes just __syncwarp and the block barrier order loads and stores. ThreadSanitizer then reports any shared or
-// global access that a kernel leaves unordered. Full-warp masks only; a block's threads are whole warps.
+// global access that a kernel leaves unordered. Full-warp masks only; a block's threads are whole warps. Blocks of more
+// than 256 threads keep shim.h's collectives on barriers: a thousand spinning threads take seconds.
 #pragma once
 #define __shfl_sync shim_shfl_sync
 #define __shfl_up_sync shim_shfl_up_sync
@@ -76,24 +77,35 @@ template <class Pred> inline unsigned Lanes(uint64_t v, Pred pred)
 }
 }  // namespace emu
 
-template <class T> inline T __shfl_sync(unsigned, T v, int src) { return emu::Exchange(v, src & 31, true); }
-template <class T> inline T __shfl_up_sync(unsigned, T v, unsigned d)
+namespace emu {
+inline bool Large() { return blockDim.x > 256; }
+}  // namespace emu
+
+template <class T> inline T __shfl_sync(unsigned m, T v, int src)
+{
+	return emu::Large() ? shim_shfl_sync(m, v, src) : emu::Exchange(v, src & 31, true);
+}
+template <class T> inline T __shfl_up_sync(unsigned m, T v, unsigned d)
 {
 	const int s = emu::lane() - static_cast<int>(d);
-	return emu::Exchange(v, s, s >= 0);
+	return emu::Large() ? shim_shfl_up_sync(m, v, d) : emu::Exchange(v, s, s >= 0);
 }
-template <class T> inline T __shfl_down_sync(unsigned, T v, unsigned d)
+template <class T> inline T __shfl_down_sync(unsigned m, T v, unsigned d)
 {
 	const int s = emu::lane() + static_cast<int>(d);
-	return emu::Exchange(v, s, s <= 31);
+	return emu::Large() ? shim_shfl_down_sync(m, v, d) : emu::Exchange(v, s, s <= 31);
 }
-template <class T> inline T __shfl_xor_sync(unsigned, T v, int m) { return emu::Exchange(v, emu::lane() ^ m, true); }
-inline unsigned __ballot_sync(unsigned, int pred)
+template <class T> inline T __shfl_xor_sync(unsigned m, T v, int x)
 {
-	return emu::Lanes(pred ? 1u : 0u, [](uint64_t v) { return v != 0; });
+	return emu::Large() ? shim_shfl_xor_sync(m, v, x) : emu::Exchange(v, emu::lane() ^ x, true);
 }
-template <class T> inline unsigned __match_any_sync(unsigned, T v)
+inline unsigned __ballot_sync(unsigned m, int pred)
 {
+	return emu::Large() ? shim_ballot_sync(m, pred) : emu::Lanes(pred ? 1u : 0u, [](uint64_t v) { return v != 0; });
+}
+template <class T> inline unsigned __match_any_sync(unsigned m, T v)
+{
+	if (emu::Large()) { return shim_match_any_sync(m, v); }
 	const uint64_t mine = emu::bits(v);
 	return emu::Lanes(mine, [mine](uint64_t x) { return x == mine; });
 }

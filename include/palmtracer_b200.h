@@ -7,6 +7,10 @@
  * ABI; bad input yields 0 / no output, failed fits yield the usual -1 sentinel rows). All buffers are caller-owned
  * HOST memory; the library keeps no pointer after a call returns.
  *
+ * Memory kept between calls: each engine of a device's pool (one per concurrent call, PTB_MAX_ENGINES at most) keeps the
+ * workspace and staging buffers of its largest call and a 16 MiB pinned ring, and each device a scratch pool of at most
+ * 1 GiB. When one of the library's own allocations finds no room, the scratch pool is given back first.
+ *
  * Layouts (lib/Constants.hpp:31-64):
  *   input       uint16 [planes][height][width], x fastest
  *   output      float64 rows of 18 columns: Id, Plane, Index, Channel, X, Y, Z, Integrated intensity, SigmaX, SigmaY,

@@ -185,7 +185,10 @@ bool AllowSmemOnDevice(const void* kernel, size_t bytes, std::atomic<uint64_t>& 
 	return true;
 }
 
-cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
+namespace {
+
+// The current device's scratch pool (made on first use when `make` is set), or null.
+cudaError_t ScratchPool(bool make, cudaMemPool_t* pool)
 {
 	constexpr int kDevices = 64;
 	static std::mutex mu;
@@ -193,22 +196,38 @@ cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
 	int dev = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess || dev < 0 || dev >= kDevices) { return e != cudaSuccess ? e : cudaErrorInvalidDevice; }
-	cudaMemPool_t pool = nullptr;
-	{
-		std::lock_guard<std::mutex> lock(mu);
-		if (pools[dev] == nullptr) {
-			cudaMemPoolProps props{};
-			props.allocType = cudaMemAllocationTypePinned;
-			props.location.type = cudaMemLocationTypeDevice;
-			props.location.id = dev;
-			e = cudaMemPoolCreate(&pools[dev], &props);
-			uint64_t keep = kScratchKeep;
-			if (e == cudaSuccess) { e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep); }
-			if (e != cudaSuccess) { return e; }
-		}
-		pool = pools[dev];
+	std::lock_guard<std::mutex> lock(mu);
+	if (pools[dev] == nullptr && make) {
+		cudaMemPoolProps props{};
+		props.allocType = cudaMemAllocationTypePinned;
+		props.location.type = cudaMemLocationTypeDevice;
+		props.location.id = dev;
+		e = cudaMemPoolCreate(&pools[dev], &props);
+		uint64_t keep = kScratchKeep;
+		if (e == cudaSuccess) { e = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep); }
+		if (e != cudaSuccess) { return e; }
 	}
-	return cudaMallocFromPoolAsync(p, bytes, pool, st);
+	*pool = pools[dev];
+	return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st)
+{
+	cudaMemPool_t pool = nullptr;
+	const cudaError_t e = ScratchPool(true, &pool);
+	return e != cudaSuccess ? e : cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
+cudaError_t DeviceAlloc(void** p, size_t bytes)
+{
+	const cudaError_t e = cudaMalloc(p, bytes);
+	cudaMemPool_t pool = nullptr;
+	if (e != cudaErrorMemoryAllocation || ScratchPool(false, &pool) != cudaSuccess || !pool) { return e; }
+	cudaGetLastError();
+	if (const cudaError_t t = cudaMemPoolTrimTo(pool, 0); t != cudaSuccess) { return t; }
+	return cudaMalloc(p, bytes);
 }
 
 namespace {
@@ -596,14 +615,14 @@ bool Engine::Reserve(int H, int W, int B, uint32_t rowsCap, int slots)
 	const size_t need = PlanWorkspace(probe, H, W, B, rowsCap, nullptr);
 	if (need > poolBytes_) {
 		if (pool_) { cudaFree(pool_); pool_ = nullptr; poolBytes_ = 0; }
-		if (!PTB_CUDA(cudaMalloc(&pool_, need))) { return false; }
+		if (!PTB_CUDA(DeviceAlloc(&pool_, need))) { return false; }
 		poolBytes_ = need;
 	}
 	PlanWorkspace(ws_, H, W, B, rowsCap, static_cast<char*>(pool_));
 	if (slots > 1) {
 		if (need > pool1Bytes_) {
 			if (pool1_) { cudaFree(pool1_); pool1_ = nullptr; pool1Bytes_ = 0; }
-			if (!PTB_CUDA(cudaMalloc(&pool1_, need))) { return false; }
+			if (!PTB_CUDA(DeviceAlloc(&pool1_, need))) { return false; }
 			pool1Bytes_ = need;
 		}
 		PlanWorkspace(ws1_, H, W, B, rowsCap, static_cast<char*>(pool1_));
@@ -615,7 +634,7 @@ bool Engine::ReserveImage(size_t bytes)
 {
 	if (bytes <= imgBytes_) { return true; }
 	if (img_) { cudaFree(img_); img_ = nullptr; imgBytes_ = 0; }
-	if (!PTB_CUDA(cudaMalloc(&img_, bytes))) { return false; }
+	if (!PTB_CUDA(DeviceAlloc(&img_, bytes))) { return false; }
 	imgBytes_ = bytes;
 	return true;
 }
@@ -1238,7 +1257,7 @@ bool Engine::UploadSpline(FitParams& fp, const double* table)
 	const size_t bytes = fp.mode == kMleSpline ? 3 * raw : 2 * raw;
 	if (bytes > splineBytes_) {
 		if (spline_) { cudaFree(spline_); spline_ = nullptr; splineBytes_ = 0; }
-		if (!PTB_CUDA(cudaMalloc(&spline_, bytes))) { return false; }
+		if (!PTB_CUDA(DeviceAlloc(&spline_, bytes))) { return false; }
 		splineBytes_ = bytes;
 	}
 	double* given = static_cast<double*>(spline_);

@@ -72,6 +72,10 @@ void CountLaunch(uint64_t n = 1);
 constexpr size_t kScratchKeep = 1ull << 30;
 cudaError_t ScratchAlloc(void** p, size_t bytes, cudaStream_t st);
 
+// Device memory that an engine or the server keeps (cudaMalloc). When the device has no room, what the scratch pool keeps is
+// given back first.
+cudaError_t DeviceAlloc(void** p, size_t bytes);
+
 // Allows a kernel `bytes` of dynamic shared memory on the current device, where the runtime keeps that setting: asked for
 // once per device (`devices`, a static of the launch: the devices that have it).
 bool AllowSmemOnDevice(const void* kernel, size_t bytes, std::atomic<uint64_t>& devices);

@@ -168,7 +168,7 @@ private:
 			if (cands_) { cudaFree(cands_); cands_ = nullptr; }
 			if (rows_) { cudaFree(rows_); rows_ = nullptr; }
 			capacity_ = 0;
-			if (!PTB_CUDA(cudaMalloc(&cands_, cap * sizeof(Cand))) || !PTB_CUDA(cudaMalloc(&rows_, cap * kCols * sizeof(double)))) {
+			if (!PTB_CUDA(DeviceAlloc(&cands_, cap * sizeof(Cand))) || !PTB_CUDA(DeviceAlloc(&rows_, cap * kCols * sizeof(double)))) {
 				return false;
 			}
 			capacity_ = cap;

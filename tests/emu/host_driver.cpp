@@ -103,6 +103,25 @@ void SecondDevice()
 	cudaSetDevice(0);
 }
 
+// Scratch that the library keeps between calls is given back when another of its allocations needs the memory.
+void KeptScratch()
+{
+	const uint64_t H = 1000, W = 1000, n = 250000;
+	const uint64_t small = 1, large = 30;  // planes: 2 and 60 MB
+	std::vector<uint16_t> stack(H * W * large, 100);
+	std::vector<double> pos(n * 6, 1.0), rows(n * 18);
+	fake::limit = 100 << 20;
+	auto fit = [&](uint64_t points, uint64_t planes) {
+		return Fitting(stack.data(), pos.data(), points, rows.data(), rows.size(), H, W, planes, 2, kParams);
+	};
+	Expect(fit(n, small) == n * 18, "Fitting of many points");
+	const size_t kept = fake::used[0];
+	Expect(kept > (40u << 20), "scratch is kept");
+	Expect(fit(5, large) == 5 * 18, "Fitting on a large stack");
+	Expect(fake::used[0] < kept + (30u << 20), "scratch was given back for it");
+	Expect(fit(5, large) == 5 * 18, "Fitting afterwards");
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -112,6 +131,7 @@ int main(int argc, char** argv)
 		else if (!std::strcmp(argv[i], "null")) { NullBuffers(); }
 		else if (!std::strcmp(argv[i], "fork")) { ForkedChild(); }
 		else if (!std::strcmp(argv[i], "devices")) { SecondDevice(); }
+		else if (!std::strcmp(argv[i], "scratch")) { KeptScratch(); }
 		else { return 2; }
 	}
 	return failures ? 1 : 0;

@@ -28,3 +28,8 @@ def test_second_device(driver):
     """A process that calls the library with one device current and then with another: the kernels that take more than
     48 KB of shared memory are allowed it on both."""
     assert hostcode.run(driver, "devices") == 0
+
+
+def test_kept_scratch_makes_room(driver):
+    """A device with little memory left: scratch kept from an earlier call does not make a later call fail."""
+    assert hostcode.run(driver, "scratch") == 0

@@ -122,6 +122,19 @@ void KeptScratch()
 	Expect(fit(5, large) == 5 * 18, "Fitting afterwards");
 }
 
+// Chunks of a nine-frame host stack under the budget and chunk slots of the environment.
+void Chunks(uint64_t want)
+{
+	const uint64_t H = 256, W = 256, Z = 9;
+	std::vector<uint16_t> stack(H * W * Z, 100);
+	std::vector<double> rows((H * W / 5 + 1) * Z * 18);
+	uint64_t counts[3] = {};
+	Localization(stack.data(), rows.data(), rows.size(), H, W, Z, 10.0, 0.0, 0, kParams);
+	PTB_GraphStats(counts, 3);
+	Expect(!*PTB_LastError() && counts[0] + counts[1] + counts[2] == want, "chunks");
+	std::printf("     %llu\n", static_cast<unsigned long long>(counts[0] + counts[1] + counts[2]));
+}
+
 }  // namespace
 
 int main(int argc, char** argv)
@@ -132,6 +145,7 @@ int main(int argc, char** argv)
 		else if (!std::strcmp(argv[i], "fork")) { ForkedChild(); }
 		else if (!std::strcmp(argv[i], "devices")) { SecondDevice(); }
 		else if (!std::strcmp(argv[i], "scratch")) { KeptScratch(); }
+		else if (!std::strcmp(argv[i], "chunks") && i + 1 < argc) { Chunks(static_cast<uint64_t>(std::atoi(argv[++i]))); }
 		else { return 2; }
 	}
 	return failures ? 1 : 0;

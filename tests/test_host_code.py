@@ -33,3 +33,12 @@ def test_second_device(driver):
 def test_kept_scratch_makes_room(driver):
     """A device with little memory left: scratch kept from an earlier call does not make a later call fail."""
     assert hostcode.run(driver, "scratch") == 0
+
+
+@pytest.mark.parametrize("budget, slots, chunks", [("8", "1", 9), ("40", "1", 5), ("76", "2", 5)])
+def test_chunks_of_a_budget(driver, monkeypatch, budget, slots, chunks):
+    """Budgets in MB at which nine 256 x 256 frames come as single frames, and as 1, 2, 3, 2, 1 (three per chunk, the first
+    chunk split and the end shrinking)."""
+    monkeypatch.setenv("PTB_WORKSPACE_MB", budget)
+    monkeypatch.setenv("PTB_CHUNK_SLOTS", slots)
+    assert hostcode.run(driver, "chunks", str(chunks)) == 0

@@ -147,16 +147,16 @@ def mad_threshold_gpu(lib, frame):
 
 
 def reference_threshold(frame):
-    """The MAD threshold of a frame's W1 plane computed by the reference build's own Wavelett (the oracle port when
-    the build is absent), for the reference arm: the same value as the GPU arm's, since the planes are bit-exact."""
+    """The MAD threshold of a frame's W1 plane computed by the reference build's own Wavelett, for the reference arm: the
+    same value as the GPU arm's, since the planes are bit-exact."""
     import synth
-    from oracle.oracle import reference, OracleLib
-    lib = reference() or OracleLib()
-    return synth.mad_threshold(lib.wavelett(frame, 2)[0])
+    from oracle.oracle import reference
+    return synth.mad_threshold(reference().wavelett(frame, 2)[0])
 
 
 def cpu_reference_rate(frames_host, thr, seconds=10.0, threads=None):
-    """Reference CPU path (oracle/_ref, or the oracle port when the reference build is absent) on a bounded sample."""
+    """CPU path on a bounded sample: the reference's build (oracle/_ref), or, for the other arm's CPU figure alone, the oracle
+    port when there is none ("kind" says which)."""
     from oracle.oracle import reference, OracleLib
     lib = reference()
     kind = "reference"
@@ -539,6 +539,12 @@ def main():
     ap.add_argument("--no-parity", action="store_true", help="skip the parity check of the benchmark's own frames")
     ap.add_argument("--no-pageable", action="store_true", help="skip the end-to-end run from pageable host memory")
     args = ap.parse_args()
+    if args.impl == "reference":
+        from oracle.oracle import reference
+        if reference() is None:  # nothing else stands in for it
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": "no build of the reference here (its sources are absent)"}), flush=True)
+            return
     import torch
     import torch.distributed as dist
 

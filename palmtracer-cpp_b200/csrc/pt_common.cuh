@@ -148,7 +148,7 @@ struct Counters {
 	uint32_t fault;        // a kernel's bounded wait ran out (its results are void; the call fails)
 	uint32_t boxNext;      // work queue of the shared-memory group floods: next multi-label group to take
 	uint32_t nunion;       // domain pixels that join two union-find trees (listed in lab for the union pass)
-	uint32_t sorted;       // frames ordered by SortFrames
+	uint32_t sorted;       // CTAs of SortFrames that have finished (up to 16 per frame)
 	uint32_t fuseNext;     // work queue of the shared-memory basin fusions: next multi-label group to take
 	uint32_t nfuse;        // groups too large for them (listed in rfGroups, which the re-flood does not use after a fusion)
 };
@@ -159,7 +159,7 @@ enum RouteReason : int {
 	kRouteFirstTest = 1,    // a pair failed the first test where no rank test follows (segmentation mode 2)
 	kRouteRankSlots = 2,    // more frames needed the rank test than a chunk has slots
 	kRoutePairs = 3,        // the frame had more failing pairs than the rank test takes per frame
-	kRouteRankFused = 4,    // (none: the rank test comes before the fusion)
+	kRouteRankFused = 4,    // reserved: always 0, since the rank test comes before the fusion
 	kRouteRefloodSlots = 5, // failed the rank test beyond the re-flood slots or the re-flood's domain-pixel capacity
 	kRouteRefloodTest = 6   // the re-flooded labels failed the per-element rank test
 };

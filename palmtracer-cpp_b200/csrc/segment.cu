@@ -986,10 +986,17 @@ __global__ void __launch_bounds__(kFloodThreads) GroupFlood(Workspace ws, uint32
 // ---- Frame-wide flood by a warp -----------------------------------------------------------------------------------
 // A whole frame's flood (a routed frame, or every frame in strict mode) with its open entries in a 32-ary heap, its
 // first 16384 entries in shared memory: a level of a pop is one minimum over the lanes, three levels hold 32 768
-// entries, and eight lanes look at the popped pixel's neighbours while the heap is put in order. Equal keys (popped one
-// after the other; three frames in four have two equal seeds) end it, and the frame is flooded again with the binary
-// heap (FloodBinary). Bound: the serial chain of pops, about 1.5 us each (the neighbours come from L2). A 1024 x 1024
-// frame of 47 000 domain pixels takes 70 ms, with a tie 120-160 ms; one thread with the heap in global memory took 285 ms.
+// entries, and eight lanes look at the popped pixel's neighbours while the heap is put in order. Equal keys end it (three
+// frames in four have two equal seeds), and the frame is flooded again with the binary heap (FloodBinary). Bound: the
+// serial chain of pops, about 1.5 us each (the neighbours come from L2). A 1024 x 1024 frame of 47 000 domain pixels takes
+// 70 ms, with a tie 120-160 ms; one thread with the heap in global memory took 285 ms.
+//
+// A pop is compared with the one before it, which finds every tie, because keys leave the heap in non-decreasing order: let
+// p's pop push q. From q a path of rising W1 leads to a seed (every local maximum of the domain is one); take its first
+// labelled pixel. That is p, or it is open: its predecessor on the path is unlabelled, so it has not been popped, nor was it
+// a closed seed. Either way its key is not below p's, and q's is not below that: q's W1 is lower, its aging term at least as
+// large, and rounding is monotone. The second flood of a basin fusion starts from one seed per basin, where such a path may
+// end at a maximum without a label: it must not be done here.
 constexpr size_t kFrameHeapBytes = kFrameHeap * (sizeof(unsigned long long) + sizeof(uint32_t));
 constexpr unsigned long long kNoKey = ~0ull;
 
@@ -1870,7 +1877,7 @@ __global__ void SuspectCount(Workspace ws)
 }
 
 // Step 3: the rank test of every counted pair; a frame that fails it is flooded again per component with estimated
-// frame-wide aging.
+// frame-wide aging. (The unused argument is kept for the CPU emulation of one frame.)
 __global__ void SuspectCheck(Workspace ws, int)
 {
 	PTB_AFTER_PREVIOUS();

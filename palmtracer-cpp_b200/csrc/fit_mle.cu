@@ -1347,7 +1347,8 @@ __global__ void __launch_bounds__(kThreads, MODEL == 6 && L == 1 ? 8 : 0) MlePol
 // for L = 1: per thread the FP64 column factors (3 roi doubles), lane-interleaved; L > 1: per group the column and row
 // factors (modes 6, 7). Modes 6 and 8 are held to 128 registers (8 blocks of 64 threads per SM), which they fit without
 // spilling; mode 7 keeps the compiler's own allocation (a bound spills it). Mode 8, 94 152 ROIs of 13 x 13: 2.12 ms with
-// one thread per ROI, 0.81 with 8 lanes (4: 0.84, 16: 0.85), 0.69 with the bound. Modes 6 and 7 are bound by their FP64
+// one thread per ROI, 0.81 with 8 lanes (4: 0.84, 16: 0.85), 0.69 with the bound. The lanes' partial sums, joined by
+// shuffles, are closer to long double than one thread's (CRLB of z, p99 over 1 109 fits: 2-4e-12 against 0.9-1.8e-11). Modes 6 and 7 are bound by their FP64
 // work and 4 lanes, which repeat the 5 x 5 inverse, are no faster (mode 6 0.79 -> 1.07 ms, mode 7 0.38 -> 0.36 ms).
 template <int MODEL, int L>
 __global__ void __launch_bounds__(kThreads, MODEL == 7 ? 0 : 8) MleFinalKernel(FitImages fi,

@@ -213,9 +213,7 @@ __device__ __forceinline__ bool LocateRoi(const uint16_t* frame, int H, int W, c
 	const unsigned long long ux = nonneg ? static_cast<unsigned long long>(cd.x) : 0ull;
 	const unsigned long long uy = nonneg ? static_cast<unsigned long long>(cd.y) : 0ull;
 	const unsigned long long h = static_cast<unsigned long long>(fp.half);
-	if (!nonneg || h > ux || ux >= static_cast<unsigned long long>(W) - h || h > uy || uy >= static_cast<unsigned long long>(H) - h) {
-		return false;
-	}
+	if (!nonneg || !RoiInside(ux, uy, fp.half, H, W)) { return false; }
 	R.base = frame + static_cast<long long>(uy - h) * W + static_cast<long long>(ux - h);
 	R.W = W;
 	R.roi = fp.roi;

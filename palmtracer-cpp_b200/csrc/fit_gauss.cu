@@ -335,7 +335,7 @@ __device__ void FitOne(const uint16_t* frame, int H, int W, const FitParams& fp,
 	const unsigned long long ux = nonneg ? static_cast<unsigned long long>(cd.x) : 0ull;
 	const unsigned long long uy = nonneg ? static_cast<unsigned long long>(cd.y) : 0ull;
 	const unsigned long long h = static_cast<unsigned long long>(half);
-	if (!nonneg || h > ux || ux >= static_cast<unsigned long long>(W) - h || h > uy || uy >= static_cast<unsigned long long>(H) - h) {
+	if (!nonneg || !RoiInside(ux, uy, half, H, W)) {
 		StoreRow(row, MODE, cd.intensity, cd.surf, cd.x, cd.y, 0, -1, -1, -1, -1, -1, -1, -1);
 		if (cleanOut) { *cleanOut = true; }
 		return;

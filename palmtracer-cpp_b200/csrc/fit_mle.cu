@@ -701,9 +701,7 @@ __device__ __forceinline__ bool Locate(const FitImages& fi, const MleParams& mp,
 	r.ux = nonneg ? static_cast<unsigned long long>(cd.x) : 0ull;
 	r.uy = nonneg ? static_cast<unsigned long long>(cd.y) : 0ull;
 	const unsigned long long hh = static_cast<unsigned long long>(mp.half);
-	if (!nonneg || hh > r.ux || r.ux >= static_cast<unsigned long long>(W) - hh || hh > r.uy || r.uy >= static_cast<unsigned long long>(H) - hh) {
-		return false;
-	}
+	if (!nonneg || !RoiInside(r.ux, r.uy, mp.half, H, W)) { return false; }
 	r.x0 = cd.x - static_cast<double>(r.ux);
 	r.y0 = cd.y - static_cast<double>(r.uy);
 	r.base = f.img + static_cast<long long>(cd.frame) * f.N + static_cast<long long>(r.uy - hh) * W + static_cast<long long>(r.ux - hh);
@@ -1348,8 +1346,9 @@ __global__ void __launch_bounds__(kThreads, MODEL == 6 && L == 1 ? 8 : 0) MlePol
 // factors (modes 6, 7). Modes 6 and 8 are held to 128 registers (8 blocks of 64 threads per SM), which they fit without
 // spilling; mode 7 keeps the compiler's own allocation (a bound spills it). Mode 8, 94 152 ROIs of 13 x 13: 2.12 ms with
 // one thread per ROI, 0.81 with 8 lanes (4: 0.84, 16: 0.85), 0.69 with the bound. The lanes' partial sums, joined by
-// shuffles, are closer to long double than one thread's (CRLB of z, p99 over 1 109 fits: 2-4e-12 against 0.9-1.8e-11). Modes 6 and 7 are bound by their FP64
-// work and 4 lanes, which repeat the 5 x 5 inverse, are no faster (mode 6 0.79 -> 1.07 ms, mode 7 0.38 -> 0.36 ms).
+// shuffles, are closer to long double than one thread's (CRLB of z, p99 over 1 109 fits: 2-4e-12 against 0.9-1.8e-11).
+// Modes 6 and 7 are bound by their FP64 work and 4 lanes, which repeat the 5 x 5 inverse, are no faster (mode 6 0.79 ->
+// 1.07 ms, mode 7 0.38 -> 0.36 ms).
 template <int MODEL, int L>
 __global__ void __launch_bounds__(kThreads, MODEL == 7 ? 0 : 8) MleFinalKernel(FitImages fi,
                                                            const Cand* __restrict__ cands, const uint32_t* nptr, uint32_t nconst,

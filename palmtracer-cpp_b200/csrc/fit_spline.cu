@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * kWarps, 3) SplineFitKernel(const uint16_t
 		const unsigned long long ux = nonneg ? static_cast<unsigned long long>(cd.x) : 0ull;
 		const unsigned long long uy = nonneg ? static_cast<unsigned long long>(cd.y) : 0ull;
 		const unsigned long long h = static_cast<unsigned long long>(hh);
-		if (!nonneg || h > ux || ux >= static_cast<unsigned long long>(W) - h || h > uy || uy >= static_cast<unsigned long long>(H) - h) {
+		if (!nonneg || !RoiInside(ux, uy, hh, H, W)) {
 			StoreRow(row, cd.intensity, cd.surf, cd.x, cd.y, 0, -1, -1, -1, -1, true);
 			continue;
 		}

@@ -259,6 +259,15 @@ struct Geometry {
 	FastDiv divN, divW;
 };
 
+// True when the ROI of 2 half + 1 pixels around (ux, uy) lies in the frame (the reference's border test, Fitting.cpp). No
+// such position exists where the frame is narrower than the half ROI: W - half must not wrap.
+__host__ __device__ __forceinline__ bool RoiInside(unsigned long long ux, unsigned long long uy, int half, int H, int W)
+{
+	const unsigned long long h = static_cast<unsigned long long>(half), w = static_cast<unsigned long long>(W),
+	                         r = static_cast<unsigned long long>(H);
+	return h <= ux && h <= uy && w > h && r > h && ux < w - h && uy < r - h;
+}
+
 // Re-flood slots of a chunk.
 __host__ __device__ __forceinline__ uint32_t RefloodSlots(const Geometry& g)
 {

@@ -147,11 +147,13 @@ def mad_threshold_gpu(lib, frame):
 
 
 def reference_threshold(frame):
-    """The MAD threshold of a frame's W1 plane computed by the reference build's own Wavelett, for the reference arm: the
-    same value as the GPU arm's, since the planes are bit-exact."""
+    """The MAD threshold of a frame's W1 plane computed by the reference build's own Wavelett, for the reference arm (the
+    oracle port's where there is no build, for the tests): the same value as the GPU arm's, since the planes are
+    bit-exact."""
     import synth
-    from oracle.oracle import reference
-    return synth.mad_threshold(reference().wavelett(frame, 2)[0])
+    from oracle.oracle import reference, OracleLib
+    lib = reference() or OracleLib()
+    return synth.mad_threshold(lib.wavelett(frame, 2)[0])
 
 
 def cpu_reference_rate(frames_host, thr, seconds=10.0, threads=None):
